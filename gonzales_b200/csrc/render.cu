@@ -745,8 +745,7 @@ __device__ void camera_ray(const SceneConst &sc, uint32_t px, uint32_t py, uint3
         gaussian_sample_1d(u0, sc.filter_radius, sc.filter_sigma, dx, denx);
         gaussian_sample_1d(u1, sc.filter_radius, sc.filter_sigma, dy, deny);
         const float fx = (float)px + 0.5f + dx, fy = (float)py + 0.5f + dy;
-        float l0, l1;
-        zs_get2d(sc.zs, z, l0, l1);  // lens sample (drawn also by a pinhole)
+        const ZSlot lens = zs_take(z, 2);  // a pinhole takes the lens sample's dimensions too
         // raster -> screen -> camera -> world
         const float scx = sc.sx0 + fx / (float)sc.width * (sc.sx1 - sc.sx0);
         const float scy = sc.sy1 - fy / (float)sc.height * (sc.sy1 - sc.sy0);
@@ -757,8 +756,9 @@ __device__ void camera_ray(const SceneConst &sc, uint32_t px, uint32_t py, uint3
                 // the origin moves to the lens point; as written the new
                 // direction is taken from the pinhole origin, so it keeps the
                 // pinhole direction (renormalised after scaling to the focal plane)
-                float lx, ly;
-                concentric_disk(l0, l1, lx, ly);
+                float l[2], lx, ly;
+                zs_draw<2>(sc.zs, z, lens, l);
+                concentric_disk(l[0], l[1], lx, ly);
                 lx = sc.lens_radius * lx;
                 ly = sc.lens_radius * ly;
                 const float ft = sc.focal_distance / dcam.z;
@@ -775,6 +775,7 @@ __device__ void camera_ray(const SceneConst &sc, uint32_t px, uint32_t py, uint3
 // to the scene whose [path_begin, next path_begin) holds it; within the scene
 // path q is sample q % spp of pixel q / spp.
 __global__ void k_generate(Wave w) {
+        zs_block_init();
         const uint32_t count = wave_count(w);
         const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
         if (threadIdx.x == 0 && blockIdx.x == 0) {
@@ -819,6 +820,7 @@ __global__ void k_generate(Wave w) {
 // loops: Ray_C records (origin, direction), ray weights and pixel indices.
 __global__ void k_camera_rays(SceneConst sc, uint64_t first, uint64_t n, float *rays6, float *weight,
                               int32_t *pixel_out) {
+        zs_block_init();
         const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
         if (i >= n) return;
         const uint64_t q = first + i;
@@ -999,10 +1001,11 @@ __device__ void shade_generic(const Wave &w, const DevScene &s, const SceneConst
                                 w.sh_contrib[q] = make_float4(c.x, c.y, c.z, 0.0f);
                         }
                 }
-                float v0, v1, v2;
-                zs_get3d(sc.zs, z, v0, v1, v2);
+                const ZSlot probe_slot = zs_take(z, 3);
                 if (sc.mis_corrected || chose_env) {
-                        const BsdfS bs = bmat_sample<K>(bm, wo_l, v0, v1, v2);
+                        float v[3];
+                        zs_draw<3>(sc.zs, z, probe_slot, v);
+                        const BsdfS bs = bmat_sample<K>(bm, wo_l, v[0], v[1], v[2]);
                         const float pdf_b = bs.pdf;
                         const V3 wi = fr.to_world(bs.wi);
                         const V3 est = bs.f * fabsf(dot(wi, ns));
@@ -1035,8 +1038,14 @@ __device__ void shade_generic(const Wave &w, const DevScene &s, const SceneConst
                                 }
                         }
                 }
-                zs_get3d(sc.zs, z, v0, v1, v2);
-                const BsdfS bs = bmat_sample<K>(bm, wo_l, v0, v1, v2);
+                // the last vertex of a path has no continuation
+                if (bounce + 1 >= sc.max_depth) {
+                        w.L[path] = make_float4(L.x, L.y, L.z, 0.0f);
+                        return;
+                }
+                float v[3];
+                zs_draw<3>(sc.zs, z, zs_take(z, 3), v);
+                const BsdfS bs = bmat_sample<K>(bm, wo_l, v[0], v[1], v[2]);
                 const float pdf_c = bs.pdf;
                 if (pdf_c == 0.0f || isnan(pdf_c)) {
                         alive = false;
@@ -1053,7 +1062,7 @@ __device__ void shade_generic(const Wave &w, const DevScene &s, const SceneConst
                                 else
                                         thr = thr * (1.0f / (1.0f - qq));
                         }
-                        if (alive && bounce + 1 < sc.max_depth) {
+                        if (alive) {
                                 const int nxt = cur ^ 1;
                                 const uint32_t q = queue_slot(w.counts + nxt);
                                 store_ray(w.q_ray[nxt], q, o, kInf, wi, sc.root);
@@ -1137,11 +1146,11 @@ __device__ void shade_medium(const Wave &w, const DevScene &s, const SceneConst 
                         w.sh_id[q] = path;
                         w.sh_contrib[q] = make_float4(c.x, c.y, c.z, 0.0f);
                 }
-                float v0, v1;
-                zs_get2d(sc.zs, z, v0, v1);
+                const ZSlot probe_slot = zs_take(z, 2);
                 if (sc.mis_corrected || chose_env) {
-                        float value;
-                        const V3 wi = hg_sample(wo, g, v0, v1, value);
+                        float v[2], value;
+                        zs_draw<2>(sc.zs, z, probe_slot, v);
+                        const V3 wi = hg_sample(wo, g, v[0], v[1], value);
                         if (value > 0.0f) {
                                 float light_density = 0.0f;
                                 if (chose_env) {
@@ -1172,6 +1181,11 @@ __device__ void shade_medium(const Wave &w, const DevScene &s, const SceneConst 
                         }
                 }
         }
+        // the last vertex of a path has no continuation
+        if (bounce + 1 >= sc.max_depth) {
+                w.L[path] = make_float4(L.x, L.y, L.z, 0.0f);
+                return;
+        }
         float v0, v1;
         zs_get2d(sc.zs, z, v0, v1);
         float value;
@@ -1184,7 +1198,7 @@ __device__ void shade_medium(const Wave &w, const DevScene &s, const SceneConst 
                 else
                         thr = thr * (1.0f / (1.0f - qq));
         }
-        if (alive && bounce + 1 < sc.max_depth) {
+        if (alive) {
                 const int nxt = cur ^ 1;
                 const uint32_t q = queue_slot(w.counts + nxt);
                 store_ray(w.q_ray[nxt], q, p, kInf, wi, sc.root);
@@ -1214,6 +1228,7 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
                                       : kKind == kShadeDiffuse                                    ? 7
                                                                                                   : 6)
     k_shade(Wave w, DevScene s, int bounce, int cur, int sorted) {
+        zs_block_init();
         const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
         uint32_t i;
         if (kKind >= kShadeDielectric) {
@@ -1422,10 +1437,12 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
                 // chosen light's density along it: an environment light answers
                 // from its map; an area light, as written, answers 0 (queried with
                 // tHit = 0), so that strategy is traced only for corrected MIS.
-                float v0, v1, v2;
-                zs_get3d(sc.zs, z, v0, v1, v2);
+                // A diffuse BSDF uses two of a sample's three numbers.
+                const ZSlot probe_slot = zs_take(z, 3);
                 if (sc.mis_corrected || chose_env) {
-                        V3 wi_l = cosine_hemisphere(v0, v1);
+                        float v[2];
+                        zs_draw<2>(sc.zs, z, probe_slot, v);
+                        V3 wi_l = cosine_hemisphere(v[0], v[1]);
                         if (wo_l.z < 0.0f) wi_l.z = -wi_l.z;
                         const float pdf_b = (wo_l.z * wi_l.z > 0.0f) ? fabsf(wi_l.z) / kPi : 0.0f;
                         const V3 wi = fr.to_world(wi_l);
@@ -1461,8 +1478,14 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
                         }
                 }
                 // ---- continuation (bsdf.sampleWorldSpace, :358-369)
-                zs_get3d(sc.zs, z, v0, v1, v2);
-                V3 wi_l = cosine_hemisphere(v0, v1);
+                // the last vertex of a path has none
+                if (bounce + 1 >= sc.max_depth) {
+                        w.L[path] = make_float4(L.x, L.y, L.z, 0.0f);
+                        return;
+                }
+                float v[2];
+                zs_draw<2>(sc.zs, z, zs_take(z, 3), v);
+                V3 wi_l = cosine_hemisphere(v[0], v[1]);
                 if (wo_l.z < 0.0f) wi_l.z = -wi_l.z;
                 const float pdf_c = (wo_l.z * wi_l.z > 0.0f) ? fabsf(wi_l.z) / kPi : 0.0f;
                 if (pdf_c == 0.0f || isnan(pdf_c)) {
@@ -1480,7 +1503,7 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
                                 else
                                         thr = thr * (1.0f / (1.0f - qq));
                         }
-                        if (alive && bounce + 1 < sc.max_depth) {
+                        if (alive) {
                                 const int nxt = cur ^ 1;
                                 const uint32_t q = queue_slot(w.counts + nxt);
                                 store_ray(w.q_ray[nxt], q, o, kInf, wi, sc.root);
@@ -1685,6 +1708,7 @@ struct KindList {
 // calls in `kinds` (1, 2 or 3 each), starting at dimension 0.
 __global__ void k_zsobol_fill(ZSobolConfig c, const int32_t *px, const int32_t *py, const int64_t *index, int64_t n,
                               KindList kinds, int nkinds, int per, float *out) {
+        zs_block_init();
         const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
         if (i >= n) return;
         ZSobol z;
@@ -1717,10 +1741,21 @@ gzg_status device_sobol(int dev, const uint32_t **out) {
                 const uint32_t *host = sobol_matrices(&count);
                 if (count != (size_t)kSobolDims * kSobolColumns)
                         return set_error(GZG_ERR_BAD_SCENE, "embedded Sobol table has the wrong size");
+                // the matrices, then the nibble tables made from them
+                std::vector<uint32_t> table(host, host + count);
+                table.resize(count + (size_t)kSobolDims * kSobolNibbleWords);
+                for (int d = 0; d < kSobolDims; ++d)
+                        for (int g = 0; g < 8; ++g)
+                                for (int v = 0; v < 16; ++v) {
+                                        uint32_t x = 0;
+                                        for (int b = 0; b < 4; ++b)
+                                                if ((v >> b) & 1) x ^= host[(size_t)d * kSobolColumns + 4 * g + b];
+                                        table[count + (size_t)d * kSobolNibbleWords + 16 * g + v] = x;
+                                }
                 void *p = nullptr;
-                cudaError_t e = cudaMalloc(&p, count * 4);
+                cudaError_t e = cudaMalloc(&p, table.size() * 4);
                 if (e != cudaSuccess) return set_error(GZG_ERR_OUT_OF_MEMORY, "Sobol table allocation");
-                e = cudaMemcpy(p, host, count * 4, cudaMemcpyHostToDevice);
+                e = cudaMemcpy(p, table.data(), table.size() * 4, cudaMemcpyHostToDevice);
                 if (e != cudaSuccess) return set_error(GZG_ERR_CUDA, "Sobol table upload");
                 g_sobol_dev[dev] = static_cast<const uint32_t *>(p);
         }
@@ -1732,6 +1767,7 @@ gzg_status device_sobol(int dev, const uint32_t **out) {
 ZSobolConfig make_zsobol(int64_t spp, int32_t res_x, int32_t res_y, int64_t seed, const uint32_t *matrices) {
         ZSobolConfig c{};
         c.matrices = matrices;
+        c.nibbles = matrices + (size_t)kSobolDims * kSobolColumns;
         c.seed = (uint64_t)seed;
         c.log2spp = __builtin_ctzll((uint64_t)spp);
         int64_t res = std::max(res_x, res_y);

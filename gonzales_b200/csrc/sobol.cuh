@@ -10,6 +10,9 @@ namespace gzg {
 
 constexpr int kSobolDims = 1024;
 constexpr int kSobolColumns = 52;
+// Per dimension: the xor of the first 32 matrix columns over each 4-bit group
+// of index bits, [8 groups][16 values] (512 KB for all dimensions).
+constexpr int kSobolNibbleWords = 8 * 16;
 
 struct ZSobol {
         uint64_t morton;  // (Morton(px, py) << log2spp) | sample index
@@ -18,6 +21,7 @@ struct ZSobol {
 
 struct ZSobolConfig {
         const uint32_t *matrices;  // kSobolDims x kSobolColumns
+        const uint32_t *nibbles;   // kSobolDims x kSobolNibbleWords
         uint64_t seed;             // sampler seed (1234, Sampler/Random.swift:66)
         int32_t log2spp;
         int32_t n_base4_digits;
@@ -67,94 +71,154 @@ __device__ __forceinline__ uint64_t zs_morton2(uint32_t x, uint32_t y) {
 }
 
 __device__ __forceinline__ uint64_t zs_shr(uint64_t v, int s) { return s >= 64 ? 0ull : (v >> s); }
-
-// The 24 permutations of ZSobolSampler.swift:105-112 packed two bits per
-// entry, one byte per permutation, eight bytes per word (byte p & 7 of word
-// p >> 3): perm[p][d] = (byte p >> (2 * d)) & 3.  Selected from registers
-// rather than read from a local-memory array (box-scene frame 1.429 -> 1.407 ms).
-__device__ __forceinline__ int zs_perm(int p, int digit) {
-        const uint64_t word = p < 8 ? 0xB1E19C6C78D8B4E4ull : (p < 16 ? 0x72D236C68D2D39C9ull : 0x93634B1B87271E4Eull);
-        const uint32_t entry = (uint32_t)(word >> (8 * (p & 7))) & 0xFFu;
-        return (int)((entry >> (2 * digit)) & 3u);
-}
-
 __device__ __forceinline__ uint32_t zs_shr32(uint32_t v, int s) { return s >= 32 ? 0u : (v >> s); }
 
-// getSampleIndex when the Morton index (pixel Morton code << log2 spp |
-// sample) is below 2^32 and has at most 16 base-4 digits, as for 2048 x 2048
-// pixels at up to 1024 spp: the same bits as the 64-bit form in 32-bit
-// arithmetic.  mixBits folds its argument to 32 bits by xor, so for
-// higher < 2^32, mixBits(higher ^ dim x 0x55555555) is
-// mixBits32(higher ^ fold(dim x 0x55555555)).
-__device__ __forceinline__ uint32_t zs_sample_index32(const ZSobolConfig &c, uint32_t morton, int dim) {
-        const uint64_t dmul = 0x55555555ull * (uint64_t)(int64_t)dim;
-        const uint32_t dfold = (uint32_t)(dmul & 0xFFFFFFFFull) ^ (uint32_t)(dmul >> 32);
-        uint32_t idx = 0;
-        const bool pow2 = (c.log2spp & 1) == 1;
+// The 24 permutations of ZSobolSampler.swift:105-112, two bits per entry, one
+// byte per permutation (entry d of permutation p = (byte p >> (2 * d)) & 3),
+// laid out for a 256-byte shared table indexed by the top byte b of a hash:
+// entry b is permutation b % 24, so the table repeats these six words.
+__constant__ const uint32_t kZsPermWords[6] = {0x78d8b4e4u, 0xb1e19c6cu, 0x8d2d39c9u,
+                                               0x72d236c6u, 0x87271e4eu, 0x93634b1bu};
+
+// One table per block.  64 words in 32 banks: any access pattern of a warp
+// takes at most two wavefronts.
+__device__ __forceinline__ uint32_t *zs_perm_table() {
+        __shared__ uint32_t table[64];
+        return table;
+}
+
+// Fills the block's permutation table; every thread of the block calls it
+// before any of them draws a sample or returns.
+__device__ __forceinline__ void zs_block_init() {
+        uint32_t *t = zs_perm_table();
+        for (unsigned i = threadIdx.x; i < 64u; i += blockDim.x) t[i] = kZsPermWords[i % 6u];
+        __syncthreads();
+}
+
+// A draw's dimensions: the one its hashes use, and the first matrix dimension
+// (they part only where the sampler wraps around past its last dimension).
+struct ZSlot {
+        int32_t hash, base;
+};
+// Takes the next n dimensions (get1D / get2D / get3D, ZSobolSampler.swift:
+// 203-280, advance the sampler this way).  A draw whose values are not needed
+// takes its dimensions and nothing else.
+__device__ __forceinline__ ZSlot zs_take(ZSobol &s, int n) {
+        ZSlot r;
+        r.hash = s.dim;
+        if (s.dim + (n - 1) >= kSobolDims) s.dim = 2;
+        r.base = s.dim;
+        s.dim += n;
+        return r;
+}
+
+// Whether every index of this path fits 32 bits (2048 x 2048 pixels at up to
+// 1024 spp, say): the index permutation then runs in 32-bit arithmetic and the
+// matrix products come from the nibble tables.
+__device__ __forceinline__ bool zs_fits32(const ZSobolConfig &c, const ZSobol &s) {
+        return (s.morton >> 32) == 0 && c.n_base4_digits <= 16;
+}
+
+// getSampleIndex in 64-bit arithmetic (ZSobolSampler.swift:138-166) for the
+// frames that need it, out of line: the draws' code stays small (the shade
+// kernels wait on instruction fetches as it is).
+__device__ __noinline__ uint64_t zs_index64(int log2spp, int n_base4_digits, uint64_t morton, int dim) {
+        uint64_t idx = 0;
+        const bool pow2 = (log2spp & 1) == 1;
         const int last = pow2 ? 1 : 0;
-        for (int di = c.n_base4_digits - 1; di >= last; --di) {
+        const uint64_t dmul = 0x55555555ull * (uint64_t)(int64_t)dim;
+        for (int di = n_base4_digits - 1; di >= last; --di) {
                 const int shift = 2 * di - (pow2 ? 1 : 0);
-                const int digit = (int)(zs_shr32(morton, shift) & 3u);
-                const uint32_t h = zs_mix_bits32(zs_shr32(morton, shift + 2) ^ dfold);
-                idx |= (uint32_t)zs_perm((int)((h >> 24) % 24u), digit) << shift;
+                const int digit = (int)(zs_shr(morton, shift) & 3u);
+                const uint64_t higher = zs_shr(morton, shift + 2);
+                const uint32_t e = reinterpret_cast<const uint8_t *>(zs_perm_table())[zs_mix_bits(higher ^ dmul) >> 24];
+                idx |= (uint64_t)((e >> (2 * digit)) & 3u) << shift;
         }
         if (pow2) {
                 int digit = (int)(morton & 1u);
-                const uint32_t h = zs_mix_bits32((morton >> 1) ^ dfold);
-                digit ^= (int)(h & 1u);
-                idx |= (uint32_t)digit;
-        }
-        return idx;
-}
-
-// getSampleIndex (ZSobolSampler.swift:138-166).
-__device__ __forceinline__ uint64_t zs_sample_index(const ZSobolConfig &c, const ZSobol &s) {
-        if ((s.morton >> 32) == 0 && c.n_base4_digits <= 16) return zs_sample_index32(c, (uint32_t)s.morton, s.dim);
-        uint64_t idx = 0;
-        const bool pow2 = (c.log2spp & 1) == 1;
-        const int last = pow2 ? 1 : 0;
-        const uint64_t dmul = 0x55555555ull * (uint64_t)(int64_t)s.dim;
-        for (int di = c.n_base4_digits - 1; di >= last; --di) {
-                const int shift = 2 * di - (pow2 ? 1 : 0);
-                const int digit = (int)(zs_shr(s.morton, shift) & 3u);
-                const uint64_t higher = zs_shr(s.morton, shift + 2);
-                const uint32_t h = zs_mix_bits(higher ^ dmul);
-                idx |= (uint64_t)zs_perm((int)((h >> 24) % 24u), digit) << shift;
-        }
-        if (pow2) {
-                int digit = (int)(s.morton & 1u);
-                const uint32_t h = zs_mix_bits((s.morton >> 1) ^ dmul);
+                const uint32_t h = zs_mix_bits((morton >> 1) ^ dmul);
                 digit ^= (int)(h & 1u);
                 idx |= (uint64_t)digit;
         }
         return idx;
 }
 
-// sobolSample (ZSobolSampler.swift:6-31) of N consecutive dimensions d0.. for
-// one index: the XOR of the matrix columns of the index's set bits, in one
-// scan of those bits (the N columns of a bit are independent loads).
+// sobolSample's matrix product (ZSobolSampler.swift:6-31) by scanning the
+// index bits, for indices above 32 bits.
+__device__ __noinline__ uint32_t zs_sobol64(const uint32_t *m, uint64_t index) {
+        uint32_t acc = 0;
+        while (index != 0) {
+                const int bit = __ffsll((long long)index) - 1;
+                if (bit >= kSobolColumns) break;
+                acc ^= __ldg(m + bit);
+                index &= index - 1;
+        }
+        return acc;
+}
+
+// getSampleIndex of N draws of one path at once, in 32-bit arithmetic.  Every
+// base-4 digit of the Morton index is permuted by a hash of the digits above
+// it and the draw's dimension.  mixBits folds its argument to 32 bits by xor,
+// so the argument is (digits above) ^ fold(dim x 0x55555555), and its first
+// step x ^= x >> 16 distributes over that xor: one half is shared by the N
+// draws, the other by the digits.  Only the top byte of the hash is used (its
+// last step leaves that byte alone), and it picks the permutation from the
+// block's table.  About 10 instructions per digit and draw, where hashing each
+// draw on its own with h % 24 and register-selected permutations took 28.  The
+// shade kernels are bound by integer issue, mostly the sampler's: with this, the
+// nibble tables below and no values drawn that nothing reads, the box-scene
+// frame (256 x 256, 16 spp, depth 5) went 1,387 -> 1,108 us, the adjoint step
+// 4.64 -> 3.75 ms, the two-level frame with layered materials 30.9 -> 29.3 ms.
 template <int N>
-__device__ __forceinline__ void zs_sobol_bits(const ZSobolConfig &c, uint64_t index, int d0, uint32_t acc[N]) {
-        const uint32_t *m = c.matrices + (size_t)d0 * kSobolColumns;
+__device__ __forceinline__ void zs_index32(const ZSobolConfig &c, uint32_t morton, const ZSlot (&slot)[N],
+                                           uint32_t (&idx)[N]) {
+        const uint8_t *perm = reinterpret_cast<const uint8_t *>(zs_perm_table());
+        uint32_t fold[N], mixed[N];
 #pragma unroll
-        for (int k = 0; k < N; ++k) acc[k] = 0u;
-        if ((index >> 32) == 0) {
-                uint32_t cur = (uint32_t)index;
-                while (cur != 0u) {
-                        const int bit = __ffs(cur) - 1;
+        for (int k = 0; k < N; ++k) {
+                const uint64_t dmul = 0x55555555ull * (uint64_t)(int64_t)slot[k].hash;
+                fold[k] = (uint32_t)(dmul & 0xFFFFFFFFull) ^ (uint32_t)(dmul >> 32);
+                mixed[k] = fold[k] ^ (fold[k] >> 16);
+                idx[k] = 0u;
+        }
+        const int odd = c.log2spp & 1;
+#pragma unroll 1
+        for (int shift = 2 * (c.n_base4_digits - 1) - odd; shift >= odd; shift -= 2) {
+                uint32_t above = zs_shr32(morton, shift + 2);
+                above ^= above >> 16;
+                const uint32_t sel = ((morton >> shift) & 3u) * 2u;
 #pragma unroll
-                        for (int k = 0; k < N; ++k) acc[k] ^= __ldg(m + k * kSobolColumns + bit);
-                        cur &= cur - 1u;
+                for (int k = 0; k < N; ++k) {
+                        uint32_t x = (above ^ mixed[k]) * 0x85ebca77u;
+                        x ^= x >> 13;
+                        x *= 0xc2b2ae35u;
+                        const uint32_t e = perm[x >> 24];
+                        idx[k] = idx[k] * 4u + ((e >> sel) & 3u);
                 }
-        } else {
-                uint64_t cur = index;
-                while (cur != 0) {
-                        const int bit = __ffsll((long long)cur) - 1;
-                        if (bit >= kSobolColumns) break;
+        }
+        if (odd) {
 #pragma unroll
-                        for (int k = 0; k < N; ++k) acc[k] ^= __ldg(m + k * kSobolColumns + bit);
-                        cur &= cur - 1;
-                }
+                for (int k = 0; k < N; ++k)
+                        idx[k] = idx[k] * 2u + ((morton ^ zs_mix_bits32((morton >> 1) ^ fold[k])) & 1u);
+        }
+}
+
+// sobolSample's matrix products of `dims` consecutive dimensions from base for
+// a 32-bit index: one table entry per four index bits and dimension (table
+// [dim][nibble][16], the xor of the matrix columns of the nibble's set bits),
+// where scanning the index took one column per set bit in a loop as long as
+// the warp's largest bit count.
+template <int DIMS>
+__device__ __forceinline__ void zs_sobol32(const ZSobolConfig &c, uint32_t index, int base, uint32_t (&acc)[DIMS]) {
+        const uint32_t *t = c.nibbles + (size_t)base * kSobolNibbleWords;
+#pragma unroll
+        for (int k = 0; k < DIMS; ++k) acc[k] = 0u;
+        const int bits = 2 * c.n_base4_digits - (c.log2spp & 1);
+#pragma unroll 1
+        for (int b = 0; b < bits; b += 4, t += 16) {
+                const uint32_t v = (index >> b) & 15u;
+#pragma unroll
+                for (int k = 0; k < DIMS; ++k) acc[k] ^= __ldg(t + k * kSobolNibbleWords + v);
         }
 }
 
@@ -172,6 +236,39 @@ __device__ __forceinline__ uint32_t zs_hash(const ZSobolConfig &c, int dim) {
         return zs_mix_bits((uint64_t)(int64_t)dim ^ c.seed);
 }
 
+// The DIMS values of a draw whose 32-bit index is known, or (wide) of one
+// whose index needs 64 bits.
+template <int DIMS>
+__device__ __forceinline__ void zs_values(const ZSobolConfig &c, const ZSobol &s, const ZSlot &slot, bool wide,
+                                          uint32_t index, float (&out)[DIMS]) {
+        uint32_t acc[DIMS];
+        if (wide) {
+                const uint64_t idx = zs_index64(c.log2spp, c.n_base4_digits, s.morton, slot.hash);
+#pragma unroll 1
+                for (int k = 0; k < DIMS; ++k) {
+                        const uint32_t a = zs_sobol64(c.matrices + (size_t)(slot.base + k) * kSobolColumns, idx);
+#pragma unroll
+                        for (int j = 0; j < DIMS; ++j)
+                                if (j == k) acc[j] = a;
+                }
+        } else {
+                zs_sobol32<DIMS>(c, index, slot.base, acc);
+        }
+        out[0] = zs_finish(acc[0], zs_hash(c, slot.hash));
+        if (DIMS > 1) out[DIMS > 1 ? 1 : 0] = zs_finish(acc[DIMS > 1 ? 1 : 0], 0u);
+        if (DIMS > 2) out[DIMS > 2 ? 2 : 0] = zs_finish(acc[DIMS > 2 ? 2 : 0], zs_hash(c, slot.hash + 2));
+}
+
+// The first DIMS values of a draw.
+template <int DIMS>
+__device__ __forceinline__ void zs_draw(const ZSobolConfig &c, const ZSobol &s, const ZSlot &slot, float (&out)[DIMS]) {
+        const bool wide = !zs_fits32(c, s);
+        const ZSlot one[1] = {slot};
+        uint32_t idx[1] = {0u};
+        if (!wide) zs_index32<1>(c, (uint32_t)s.morton, one, idx);
+        zs_values<DIMS>(c, s, slot, wide, idx[0], out);
+}
+
 // startPixelSample (ZSobolSampler.swift:130-136).
 __device__ __forceinline__ void zs_start(const ZSobolConfig &c, ZSobol &s, uint32_t px, uint32_t py, uint32_t index) {
         s.dim = 0;
@@ -180,39 +277,29 @@ __device__ __forceinline__ void zs_start(const ZSobolConfig &c, ZSobol &s, uint3
 
 // get1D (ZSobolSampler.swift:203-219).
 __device__ __forceinline__ float zs_get1d(const ZSobolConfig &c, ZSobol &s) {
-        const uint64_t idx = zs_sample_index(c, s);
-        const uint32_t h = zs_hash(c, s.dim);
-        if (s.dim >= kSobolDims) s.dim = 2;
-        s.dim += 1;
-        uint32_t acc[1];
-        zs_sobol_bits<1>(c, idx, s.dim - 1, acc);
-        return zs_finish(acc[0], h);
+        const ZSlot slot = zs_take(s, 1);
+        float v[1];
+        zs_draw<1>(c, s, slot, v);
+        return v[0];
 }
 
 // get2D (ZSobolSampler.swift:221-244).
 __device__ __forceinline__ void zs_get2d(const ZSobolConfig &c, ZSobol &s, float &a, float &b) {
-        const uint64_t idx = zs_sample_index(c, s);
-        const uint32_t h0 = zs_hash(c, s.dim);
-        if (s.dim + 1 >= kSobolDims) s.dim = 2;
-        s.dim += 2;
-        uint32_t acc[2];
-        zs_sobol_bits<2>(c, idx, s.dim - 2, acc);
-        a = zs_finish(acc[0], h0);
-        b = zs_finish(acc[1], 0u);
+        const ZSlot slot = zs_take(s, 2);
+        float v[2];
+        zs_draw<2>(c, s, slot, v);
+        a = v[0];
+        b = v[1];
 }
 
 // get3D (ZSobolSampler.swift:249-280).
 __device__ __forceinline__ void zs_get3d(const ZSobolConfig &c, ZSobol &s, float &a, float &b, float &d) {
-        const uint64_t idx = zs_sample_index(c, s);
-        const uint32_t h0 = zs_hash(c, s.dim);
-        const uint32_t h2 = zs_hash(c, s.dim + 2);
-        if (s.dim + 2 >= kSobolDims) s.dim = 2;
-        s.dim += 3;
-        uint32_t acc[3];
-        zs_sobol_bits<3>(c, idx, s.dim - 3, acc);
-        a = zs_finish(acc[0], h0);
-        b = zs_finish(acc[1], 0u);
-        d = zs_finish(acc[2], h2);
+        const ZSlot slot = zs_take(s, 3);
+        float v[3];
+        zs_draw<3>(c, s, slot, v);
+        a = v[0];
+        b = v[1];
+        d = v[2];
 }
 
 }  // namespace gzg
