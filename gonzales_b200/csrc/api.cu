@@ -672,6 +672,7 @@ gzg_status upload_scene(const gzg_bvh2_node *bvh2_nodes, int64_t bvh2_node_count
         d.bvh2_count = build ? 0 : bvh2_node_count;
         d.prim_count = prim_count;
         d.wide_count = (uint32_t)wide.nodes.size();
+        d.rcp_max = wide_rcp_max(wide.nodes.data(), wide.nodes.size());
 
         gzg_scene_info &info = scene->info;
         info.bvh2_nodes = build ? 0 : bvh2_node_count;
@@ -907,6 +908,7 @@ GZG_API gzg_status gzg_gpu_build_mesh_scene(const gzg_mesh_arrays *meshes, int64
         d.bvh2_count = 0;
         d.prim_count = nt;
         d.wide_count = (uint32_t)wide.nodes.size();
+        d.rcp_max = wide_rcp_max(wide.nodes.data(), wide.nodes.size());
         gzg_scene_info &info = scene->info;
         info.bvh2_nodes = 0;
         info.prims = nt;
@@ -1006,8 +1008,9 @@ GZG_API gzg_status gzg_scene_tree_cost(const gzg_scene *scene, double *cost) {
                 const int e[3] = {nd.ex, nd.ey, nd.ez};
                 double nlo[3] = {INFINITY, INFINITY, INFINITY}, nhi[3] = {-INFINITY, -INFINITY, -INFINITY};
                 for (int s = 0; s < 8; ++s) {
-                        const bool interior = (nd.imask >> s) & 1u, leaf = (nd.meta[s] & 0x80u) != 0;
-                        if (!interior && !leaf) continue;
+                        const bool interior = (nd.imask >> s) & 1u;
+                        const int tris = wide_slot_triangles(nd, s);
+                        if (!interior && tris == 0) continue;
                         double lo[3], hi[3];
                         for (int a = 0; a < 3; ++a) {
                                 const double step = std::ldexp(1.0, e[a] - 127);
@@ -1018,7 +1021,7 @@ GZG_API gzg_status gzg_scene_tree_cost(const gzg_scene *scene, double *cost) {
                         }
                         const double dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
                         const double area = 2.0 * (dx * dy + dx * dz + dy * dz);
-                        sum += interior ? area : area * (double)(((nd.meta[s] >> 5) & 3u) + 1u);
+                        sum += interior ? area : area * (double)tris;
                 }
                 if (i == 0) {
                         const double dx = nhi[0] - nlo[0], dy = nhi[1] - nlo[1], dz = nhi[2] - nlo[2];
@@ -1207,7 +1210,7 @@ static void instance_world_bounds_tree(const WideBvh &w, const float *root6, con
                 }
                 return b;
         };
-        auto used = [](const WideNode &n, int s) { return ((n.imask >> s) & 1u) || (n.meta[s] & 0x80u); };
+        auto used = [](const WideNode &n, int s) { return ((n.imask >> s) & 1u) || wide_slot_triangles(n, s) > 0; };
         if (!w.nodes.empty()) {
                 const WideNode &root = w.nodes[0];
                 for (int s = 0; s < 8; ++s) {
@@ -1463,6 +1466,7 @@ GZG_API gzg_status gzg_instanced_scene_create(gzg_scene *const *blas, int64_t bl
         if ((st = scene->upload(&zero, 1, &ew, "error word"))) return st;
         d.err = const_cast<uint32_t *>(ew);
         d.wide_count = (uint32_t)std::min<uint64_t>(steps, 0xFFFFFFFFull);
+        d.rcp_max = wide_rcp_max(nodes.data(), nodes.size());
         scene->info.wide_nodes = (int64_t)nodes.size();
         scene->info.triangles = (int64_t)(v0.size() - tlas.v0.size());
         scene->info.prims = instance_count;

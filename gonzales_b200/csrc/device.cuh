@@ -25,6 +25,9 @@ struct DevScene {
         int64_t bvh2_count;
         int64_t prim_count;
         uint32_t wide_count;
+        // Bound on |1/direction| in the wide kernels' slab tests: 2^64, or less
+        // for scenes of extents above about 2^54 (wide_rcp_max).
+        float rcp_max = 18446744073709551616.0f;
         uint32_t *err;
         unsigned long long *counters;  // optional fetch counters (nodes, triangles, rays)
         uint32_t *sched;               // persistent kernels: per-launch pull counter (zero at launch) or null

@@ -361,7 +361,7 @@ __device__ __forceinline__ double code_area(const Tree &t, int code) {
 // one child plane quantised outward on that grid.
 __device__ void axis_grid(double lo, double hi, float *p_out, int *e_out, double *margin_out, double *step_out) {
         const double mag = fmax(fabs(lo), fabs(hi));
-        double margin = ldexp(fmax(mag, hi - lo), -18);
+        double margin = ldexp(mag, -18) + ldexp(hi - lo, -15);  // as the host conversion's
         if (!(margin > 0)) margin = 1e-30;
         float p = (float)(lo - margin);
         while ((double)p > lo - margin) p = nextafterf(p, -CUDART_INF_F);
@@ -627,18 +627,20 @@ __global__ void __launch_bounds__(128) k_collapse(Tree t, const int2 *__restrict
                 const int kc = __shfl_sync(FULL, cnt, base + k);
                 if (k < n && ks >= 0 && ks < my_slot) tri_off += (uint32_t)kc;
         }
+        const uint32_t tri_bits = g8_or(cnt > 0 ? ((1u << cnt) - 1u) << (4 * my_slot) : 0u);
         if (!overflow) {
                 if (j == 0) {
                         wn[15] = (uint8_t)imask;
                         reinterpret_cast<uint32_t *>(wn)[4] = cbase;
                         reinterpret_cast<uint32_t *>(wn)[5] = tbase;
+                        reinterpret_cast<uint32_t *>(wn)[6] = wide_imask_perm(imask);
+                        reinterpret_cast<uint32_t *>(wn)[7] = tri_bits;
                 }
                 if (is_int) {
                         const uint32_t rank = (uint32_t)__popc(imask & ((1u << my_slot) - 1u));
                         next[qbase + rank] = make_int2(kid, (int)(cbase + rank));
                 }
                 if (cnt > 0) {
-                        wn[24 + my_slot] = (uint8_t)(0x80u | ((uint32_t)(cnt - 1) << 5) | tri_off);
                         for (int q = 0; q < cnt; ++q) {
                                 const uint32_t pidx = (uint32_t)(t.keys[leaves[q]] & 0xFFFFFFFFu);
                                 float4 va = t.pv0[pidx];

@@ -36,8 +36,13 @@ gzg_status wait_stream(void *stream, const char *what);
 //   bytes 16-19  child_base: node index of the first interior child; interior
 //                children are stored contiguously in slot order
 //   bytes 20-23  tri_base: first triangle record of this node's leaf children
-//   bytes 24-31  meta[s]: 0 = empty or interior; leaf = 0x80 | (count-1) << 5 | offset,
-//                triangles tri_base+offset .. +count-1 (count <= 4, offset < 32)
+//   bytes 24-27  imask_perm: imask in four slot orders, byte j holding slot s's
+//                bit at s ^ j (byte 0 is imask): the traversal takes the byte
+//                of the ray's octant instead of permuting bits per child
+//   bytes 28-31  tri_bits: four bits per slot, the low `count` of them set for a
+//                leaf of count triangles (1..4), none for an empty or interior
+//                slot; triangle records follow tri_base in bit order, so bit b's
+//                record is tri_base + popcount(tri_bits below b)
 //   bytes 32-79  qlo_x[8] qlo_y[8] qlo_z[8] qhi_x[8] qhi_y[8] qhi_z[8]:
 //                child box = p + q * 2^(e-127), rounded outward at build time
 // Slot s holds the child lying farthest toward the octant whose sign bits are
@@ -48,11 +53,30 @@ struct alignas(16) WideNode {
         uint8_t ex, ey, ez, imask;
         uint32_t child_base;
         uint32_t tri_base;
-        uint8_t meta[8];
+        uint32_t imask_perm;
+        uint32_t tri_bits;
         uint8_t qlo[3][8];
         uint8_t qhi[3][8];
 };
 static_assert(sizeof(WideNode) == 80, "wide node must be 80 bytes");
+
+// imask_perm of an interior mask.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline uint32_t wide_imask_perm(uint32_t imask) {
+        const uint32_t swap1 = ((imask & 0x55u) << 1) | ((imask >> 1) & 0x55u);
+        const uint32_t swap2 = ((imask & 0x33u) << 2) | ((imask >> 2) & 0x33u);
+        const uint32_t swap3 = ((swap1 & 0x33u) << 2) | ((swap1 >> 2) & 0x33u);
+        return imask | (swap1 << 8) | (swap2 << 16) | (swap3 << 24);
+}
+// Triangles of slot s's leaf (0: none).
+inline int wide_slot_triangles(const WideNode &n, int s) { return __builtin_popcount((n.tri_bits >> (4 * s)) & 15u); }
+
+// The largest |1/direction| the slab tests of these nodes may use (device.cuh,
+// DevScene::rcp_max): 2^64, less for trees so large that the product of a
+// grid step, that reciprocal and 2^16 would overflow.
+float wide_rcp_max(const WideNode *nodes, size_t count);
 
 // Triangle records in leaf order: three float4 streams (v0, v1, v2); v0.w holds
 // the prim index (into the uploaded prim-id array) as int32 bits.

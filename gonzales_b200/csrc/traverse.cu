@@ -6,8 +6,8 @@
 //   visit go to a short per-thread stack in shared memory laid out
 //   [depth][blockDim] so consecutive threads hit consecutive banks.  Node
 //   records are fetched as five 128-bit read-only loads; child planes are
-//   8-bit offsets turned into floats with a byte permute and one add.  Leaf
-//   triangles are tested as soon as their node is opened, in leaf order.
+//   8-bit offsets turned into floats with a byte permute.  Leaf triangles are
+//   tested as soon as their node is opened, in leaf order.
 // k_bvh2: the host's BVH2 traversed exactly as the reference's
 //   traverse_bvh2_core (kernel.mojo:223-364), one thread per ray, with the
 //   reference's slab arithmetic (kernel.mojo:171-206) in _rn intrinsics.
@@ -77,38 +77,21 @@ __device__ __forceinline__ bool chunk_next(ChunkCursor &c, uint32_t *sched, uint
         return c.cursor < n;
 }
 
-// 8-bit quantised plane -> float: 0x4B0000qq is 2^23 + q exactly.
-__device__ __forceinline__ float qbyte(uint32_t word, uint32_t sel) {
-        return __uint_as_float(__byte_perm(word, 0x4B000000u, sel)) - 8388608.0f;
+// 1/d for the wide kernels' slab tests, kept finite: beyond +-limit (2^64 unless
+// the scene is huge; zero included) it is +-limit with d's sign.  Finite
+// reciprocals keep every plane distance free of 0 * inf = NaN, which lets the
+// slab test compare float bits as integers (below).  A plane then appears at
+// distance |dx| * limit instead of beyond it, still far past any hit distance
+// of a scene with coordinates below about 1e12, so the test stays conservative.
+__device__ __forceinline__ float wide_rcp(float d, float limit) {
+        return copysignf(fminf(fabsf(__fdiv_rn(1.0f, d)), limit), d);
 }
-
-// 1/d for the wide kernels' slab tests, kept finite: |d| <= 2^-64 (zero
-// included) gives +-2^64 with d's sign.  Finite reciprocals keep every plane
-// distance free of 0 * inf = NaN, which lets the slab test compare float bits
-// as integers (below).  A plane then appears at distance |dx| * 2^64 instead of
-// beyond it, still far past any hit distance of a scene with coordinates below
-// about 1e12, so the test stays conservative.
-__device__ __forceinline__ float wide_rcp(float d) {
-        return fabsf(d) > 5.42101086e-20f ? __fdiv_rn(1.0f, d) : copysignf(1.8446744e19f, d);
-}
-
 
 // Packed FP32 pairs (sm_100a f32x2): each element rounds exactly as the
 // scalar fadd / fmaf would, two elements per instruction.
 struct F2 {
         float x, y;
 };
-__device__ __forceinline__ F2 add2(F2 a, F2 b) {
-        F2 d;
-        asm("{.reg .b64 ra, rb, rd;\n\t"
-            "mov.b64 ra, {%2, %3};\n\t"
-            "mov.b64 rb, {%4, %5};\n\t"
-            "add.rn.f32x2 rd, ra, rb;\n\t"
-            "mov.b64 {%0, %1}, rd;}"
-            : "=f"(d.x), "=f"(d.y)
-            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-        return d;
-}
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
         F2 d;
         asm("{.reg .b64 ra, rb, rc, rd;\n\t"
@@ -121,9 +104,9 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
             : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
         return d;
 }
-// Two quantised planes as 2^23 + q floats.
+// Two quantised planes as 2^15 + q floats: byte 1 of 0x470000 00 is worth q.
 __device__ __forceinline__ F2 qbytes(uint32_t wa, uint32_t wb, uint32_t sel) {
-        return F2{__uint_as_float(__byte_perm(wa, 0x4B000000u, sel)), __uint_as_float(__byte_perm(wb, 0x4B000000u, sel))};
+        return F2{__uint_as_float(__byte_perm(wa, 0x47000000u, sel)), __uint_as_float(__byte_perm(wb, 0x47000000u, sel))};
 }
 
 struct WideRay {
@@ -132,12 +115,38 @@ struct WideRay {
         uint32_t oct;  // sign bits of the inverse direction
 };
 
-// Tests the 8 child boxes of a wide node against [0, thit].  Produces the
-// interior hit mask in key order (bit (slot ^ oct)), the node's interior mask,
-// child base, and the triangle hit mask relative to tri_base.
-__device__ __forceinline__ void open_node(const uint4 *__restrict__ node, const WideRay &r, float thit,
-                                          uint32_t &node_hits, uint32_t &imask, uint32_t &child_base,
-                                          uint32_t &tri_hits, uint32_t &tri_base) {
+// What a ray hits in a wide node.
+struct NodeHits {
+        uint32_t nodes;       // interior children, bit key = slot ^ oct
+        uint32_t imask;       // the node's interior mask, by slot
+        uint32_t child_base;
+        uint32_t tris;        // triangles of the leaf children hit, as bits of tri_bits
+        uint32_t tri_base, tri_bits;
+};
+// Record of triangle bit b of a node.
+__device__ __forceinline__ uint32_t tri_record(uint32_t tri_base, uint32_t tri_bits, uint32_t b) {
+        return tri_base + __popc(tri_bits & ((1u << b) - 1u));
+}
+
+// Tests the 8 child boxes of a wide node against [0, thit].
+// The kernels are bound by instruction issue (73 % of the slots, 14 of 32 lanes
+// active on incoherent rays), and this is most of it, so it is laid out for few
+// instructions per child:
+// - A plane's byte q goes to byte 1 of a float worth 2^15 + q, and the 2^15 is
+//   folded into the per-node constant (a - 2^15 s) instead of subtracted per
+//   plane.  Rounding that constant is off by at most 2^-9 of a grid step, which
+//   the boxes' margin covers (2^-15 of the extent, twice as much), or by
+//   2^-23 of the distance, which the far planes' slack covers.
+// - The six planes of a child are three packed pairs (near x, y; far x, y; near
+//   z, far z), one f32x2 fma each.
+// - A hit child sets one constant bit per slot order (hit) and its four
+//   triangle bits (tris); interior and leaf children part after the loop, with
+//   imask_perm and tri_bits, once per node and not per child.
+// Against a subtract per plane and a per-child branch on a meta byte (us per
+// launch): 8M incoherent rays on 1,310,720 triangles 2,581 -> 2,266, 8M camera
+// rays 1,041 -> 951, 4M any-hit rays 1,036 -> 907, 2M rays through 4096
+// instances 1,572 -> 1,384.
+__device__ __forceinline__ NodeHits open_node(const uint4 *__restrict__ node, const WideRay &r, float thit) {
         const uint4 n0 = __ldg(node + 0);
         const uint4 n1 = __ldg(node + 1);
         const uint4 n2 = __ldg(node + 2);
@@ -145,9 +154,6 @@ __device__ __forceinline__ void open_node(const uint4 *__restrict__ node, const 
         const uint4 n4 = __ldg(node + 4);
         const float px = __uint_as_float(n0.x), py = __uint_as_float(n0.y), pz = __uint_as_float(n0.z);
         const uint32_t ew = n0.w;
-        imask = ew >> 24;
-        child_base = n1.x;
-        tri_base = n1.y;
         // step * rdir (exact power-of-two scaling) and the grid origin in t.
         const float sx = __uint_as_float((ew & 0xFFu) << 23) * r.rdx;
         const float sy = __uint_as_float(((ew >> 8) & 0xFFu) << 23) * r.rdy;
@@ -155,13 +161,17 @@ __device__ __forceinline__ void open_node(const uint4 *__restrict__ node, const 
         const float ax = (px - r.ox) * r.rdx;
         const float ay = (py - r.oy) * r.rdy;
         const float az = (pz - r.oz) * r.rdz;
-        // Far planes carry the relative slack 1.0000003 of the reference's
-        // tFar (kernel.mojo:204) in their per-node constants instead of one
-        // multiply per child; thit is scaled the same way once.
-        const float kSlack = 1.0000003f;
+        // Far planes carry a relative slack (the reference's tFar has 1.0000003,
+        // kernel.mojo:204) in their per-node constants instead of one multiply
+        // per child; thit is scaled the same way once.
+        const float kSlack = 1.0000006f;
         const float fsx = sx * kSlack, fsy = sy * kSlack, fsz = sz * kSlack;
         const float fax = ax * kSlack, fay = ay * kSlack, faz = az * kSlack;
-        const float thit_far = thit * kSlack;
+        const int thit_far = __float_as_int(thit * kSlack);
+        const F2 bias{-32768.0f, -32768.0f};
+        const F2 s_nxy{sx, sy}, s_fxy{fsx, fsy}, s_z{sz, fsz};
+        const F2 a_nxy = fma2(bias, s_nxy, F2{ax, ay}), a_fxy = fma2(bias, s_fxy, F2{fax, fay}),
+                 a_z = fma2(bias, s_z, F2{az, faz});
         // near/far plane words by ray sign (lo planes are near for rdir >= 0)
         const bool nx = r.oct & 1u, ny = r.oct & 2u, nz = r.oct & 4u;
         const uint32_t lx0 = n2.x, lx1 = n2.y, ly0 = n2.z, ly1 = n2.w, lz0 = n3.x, lz1 = n3.y;
@@ -172,43 +182,37 @@ __device__ __forceinline__ void open_node(const uint4 *__restrict__ node, const 
         const uint32_t fary[2] = {ny ? ly0 : hy0, ny ? ly1 : hy1};
         const uint32_t nearz[2] = {nz ? hz0 : lz0, nz ? hz1 : lz1};
         const uint32_t farz[2] = {nz ? lz0 : hz0, nz ? lz1 : hz1};
-        const uint32_t meta[2] = {n1.z, n1.w};
-        // The six planes of a child are computed as three packed pairs (near
-        // x, y; far x, y; near z, far z), one f32x2 add and one f32x2 fma per
-        // pair instead of two scalar ones, with the same rounding per plane:
-        // incoherent rays 2,848 -> 2,891 Mrays/s, coherent 6,842 -> 7,089
-        // (ray-cast workload, bit-identical hits).
-        uint32_t nh = 0, th = 0;
-        const F2 bias{-8388608.0f, -8388608.0f};
-        const F2 s_nxy{sx, sy}, a_nxy{ax, ay}, s_fxy{fsx, fsy}, a_fxy{fax, fay}, s_z{sz, fsz}, a_z{az, faz};
+        uint32_t hit = 0, tris = 0;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
                 const int w = k >> 2;
-                const uint32_t sel = (uint32_t)(k & 3) | 0x7440u;
-                const F2 tn = fma2(add2(qbytes(nearx[w], neary[w], sel), bias), s_nxy, a_nxy);
-                const F2 tf = fma2(add2(qbytes(farx[w], fary[w], sel), bias), s_fxy, a_fxy);
-                const F2 tz = fma2(add2(qbytes(nearz[w], farz[w], sel), bias), s_z, a_z);
-                const float tnx = tn.x, tny = tn.y, tnz = tz.x;
-                const float tfx = tf.x, tfy = tf.y, tfz = tz.y;
+                const uint32_t sel = 0x7404u | ((uint32_t)(k & 3) << 4);
+                const F2 tn = fma2(qbytes(nearx[w], neary[w], sel), s_nxy, a_nxy);
+                const F2 tf = fma2(qbytes(farx[w], fary[w], sel), s_fxy, a_fxy);
+                const F2 tz = fma2(qbytes(nearz[w], farz[w], sel), s_z, a_z);
                 // max(0, tn*) and min(tf*, thit) on the float bits as signed
                 // integers: order-preserving for non-negative floats; tnear is
                 // never negative, and a negative tfar (a negative integer)
                 // rejects the box either way.  No NaN occurs (finite rdir).
-                const int tnear = __vimax3_s32_relu(__float_as_int(tnx), __float_as_int(tny), __float_as_int(tnz));
-                const int tfar = __vimin3_s32(__float_as_int(tfx), __float_as_int(tfy),
-                                              min(__float_as_int(tfz), __float_as_int(thit_far)));
+                const int tnear = __vimax3_s32_relu(__float_as_int(tn.x), __float_as_int(tn.y), __float_as_int(tz.x));
+                const int tfar = __vimin3_s32(__float_as_int(tf.x), __float_as_int(tf.y),
+                                              min(__float_as_int(tz.y), thit_far));
                 if (tnear <= tfar) {
-                        const uint32_t m = (meta[w] >> (8 * (k & 3))) & 0xFFu;
-                        if ((imask >> k) & 1u) {
-                                nh |= 1u << (k ^ r.oct);
-                        } else if (m & 0x80u) {
-                                const uint32_t cnt = ((m >> 5) & 3u) + 1u;
-                                th |= ((1u << cnt) - 1u) << (m & 31u);
-                        }
+                        hit |= (1u << k) | (1u << (8 + (k ^ 1))) | (1u << (16 + (k ^ 2))) | (1u << (24 + (k ^ 3)));
+                        tris |= 15u << (4 * k);
                 }
         }
-        node_hits = nh;
-        tri_hits = th;
+        NodeHits h;
+        // the byte of the octant's low two bits, then its nibbles swapped for
+        // the third
+        const uint32_t key = ((hit & n1.z) >> ((r.oct & 3u) * 8u)) & 0xFFu;
+        h.nodes = ((key * 0x101u) >> (r.oct & 4u)) & 0xFFu;
+        h.imask = n1.z & 0xFFu;
+        h.child_base = n1.x;
+        h.tris = tris & n1.w;
+        h.tri_base = n1.y;
+        h.tri_bits = n1.w;
+        return h;
 }
 
 template <int RAYFMT, int OUTFMT, bool ANY, int STACK, int LEAF>
@@ -226,9 +230,9 @@ __global__ void __launch_bounds__(256) k_wide(DevScene s, const void *__restrict
         r.dx = in.dx;
         r.dy = in.dy;
         r.dz = in.dz;
-        r.rdx = wide_rcp(in.dx);
-        r.rdy = wide_rcp(in.dy);
-        r.rdz = wide_rcp(in.dz);
+        r.rdx = wide_rcp(in.dx, s.rcp_max);
+        r.rdy = wide_rcp(in.dy, s.rcp_max);
+        r.rdz = wide_rcp(in.dz, s.rcp_max);
         r.oct = (__float_as_uint(r.rdx) >> 31) | ((__float_as_uint(r.rdy) >> 31) << 1) |
                 ((__float_as_uint(r.rdz) >> 31) << 2);
 
@@ -241,7 +245,7 @@ __global__ void __launch_bounds__(256) k_wide(DevScene s, const void *__restrict
         // The root is key 0 of a virtual parent whose only interior slot is oct.
         uint2 group = make_uint2(s.per_ray_root ? in.root : 0u, (1u << 24) | (1u << r.oct));
         for (;;) {
-                uint32_t tri_hits = 0, tri_base = 0;
+                uint32_t tri_hits = 0, tri_base = 0, tri_bits = 0;
                 uint32_t hits = group.y >> 24;
                 if (hits) {
                         const uint32_t key = __ffs(hits) - 1;
@@ -261,16 +265,18 @@ __global__ void __launch_bounds__(256) k_wide(DevScene s, const void *__restrict
                                 atomicOr(s.err, kErrStepCap);
                                 break;
                         }
-                        uint32_t nh, nim, cb;
-                        open_node(s.wide + 5 * (size_t)node, r, thit, nh, nim, cb, tri_hits, tri_base);
+                        const NodeHits h = open_node(s.wide + 5 * (size_t)node, r, thit);
                         ++n_nodes;
-                        group = make_uint2(cb, (nh << 24) | nim);
+                        group = make_uint2(h.child_base, (h.nodes << 24) | h.imask);
+                        tri_hits = h.tris;
+                        tri_base = h.tri_base;
+                        tri_bits = h.tri_bits;
                 }
                 bool done = false;
                 while (tri_hits) {
                         const uint32_t b = __ffs(tri_hits) - 1;
                         tri_hits &= tri_hits - 1;
-                        const uint32_t ti = tri_base + b;
+                        const uint32_t ti = tri_record(tri_base, tri_bits, b);
                         ++n_tris;
                         const float4 a = __ldg(s.tv0 + ti);
                         const float4 bb = __ldg(s.tv1 + ti);
@@ -355,9 +361,9 @@ __global__ void __launch_bounds__(128, 8) k_wide_persistent(DevScene s, const vo
                                 r.dx = in.dx;
                                 r.dy = in.dy;
                                 r.dz = in.dz;
-                                r.rdx = wide_rcp(in.dx);
-                                r.rdy = wide_rcp(in.dy);
-                                r.rdz = wide_rcp(in.dz);
+                                r.rdx = wide_rcp(in.dx, s.rcp_max);
+                                r.rdy = wide_rcp(in.dy, s.rcp_max);
+                                r.rdz = wide_rcp(in.dz, s.rcp_max);
                                 r.oct = (__float_as_uint(r.rdx) >> 31) | ((__float_as_uint(r.rdy) >> 31) << 1) |
                                         ((__float_as_uint(r.rdz) >> 31) << 2);
                                 thit = in.tmax;
@@ -376,7 +382,7 @@ __global__ void __launch_bounds__(128, 8) k_wide_persistent(DevScene s, const vo
 
                 // ---- one traversal step: open one node, test its triangles
                 bool finished = false;
-                uint32_t tri_hits = 0, tri_base = 0;
+                uint32_t tri_hits = 0, tri_base = 0, tri_bits = 0;
                 uint32_t hits = group.y >> 24;
                 if (hits) {
                         const uint32_t key = __ffs(hits) - 1;
@@ -402,16 +408,18 @@ __global__ void __launch_bounds__(128, 8) k_wide_persistent(DevScene s, const vo
                                 group.y = 0u;
                                 sp = 0;
                         } else {
-                                uint32_t nh, nim, cb;
-                                open_node(s.wide + 5 * (size_t)node, r, thit, nh, nim, cb, tri_hits, tri_base);
+                                const NodeHits h = open_node(s.wide + 5 * (size_t)node, r, thit);
                                 count_lanes(s, 0);
-                                group = make_uint2(cb, (nh << 24) | nim);
+                                group = make_uint2(h.child_base, (h.nodes << 24) | h.imask);
+                                tri_hits = h.tris;
+                                tri_base = h.tri_base;
+                                tri_bits = h.tri_bits;
                         }
                 }
                 while (tri_hits) {
                         const uint32_t b = __ffs(tri_hits) - 1;
                         tri_hits &= tri_hits - 1;
-                        const uint32_t ti = tri_base + b;
+                        const uint32_t ti = tri_record(tri_base, tri_bits, b);
                         count_lanes(s, 1);
                         const float4 a = __ldg(s.tv0 + ti);
                         const float4 bb = __ldg(s.tv1 + ti);
@@ -451,10 +459,10 @@ __global__ void __launch_bounds__(128, 8) k_wide_persistent(DevScene s, const vo
         }
 }
 
-__device__ __forceinline__ void set_ray_dirs(WideRay &r) {
-        r.rdx = wide_rcp(r.dx);
-        r.rdy = wide_rcp(r.dy);
-        r.rdz = wide_rcp(r.dz);
+__device__ __forceinline__ void set_ray_dirs(WideRay &r, float limit) {
+        r.rdx = wide_rcp(r.dx, limit);
+        r.rdy = wide_rcp(r.dy, limit);
+        r.rdz = wide_rcp(r.dz, limit);
         r.oct = (__float_as_uint(r.rdx) >> 31) | ((__float_as_uint(r.rdy) >> 31) << 1) |
                 ((__float_as_uint(r.rdz) >> 31) << 2);
 }
@@ -517,7 +525,6 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced(DevScene s, const voi
         float thit = 0.0f, bu = 0.0f, bv = 0.0f;
         int prim = -1, hit_inst = -1, cur_inst = -1, sp = 0;
         uint2 group = make_uint2(0u, 0u);
-        uint32_t pend_base = 0, pend_mask = 0;
         uint32_t steps = 0;
 
         for (;;) {
@@ -536,13 +543,12 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced(DevScene s, const voi
                                 r.dx = in.dx;
                                 r.dy = in.dy;
                                 r.dz = in.dz;
-                                set_ray_dirs(r);
+                                set_ray_dirs(r, s.rcp_max);
                                 thit = in.tmax;
                                 bu = bv = 0.0f;
                                 prim = hit_inst = cur_inst = -1;
                                 sp = 0;
                                 steps = 0;
-                                pend_mask = 0;
                                 group = make_uint2(0u, (1u << 24) | (1u << r.oct));
                         }
                         const int npop = __popc(need);
@@ -553,56 +559,59 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced(DevScene s, const voi
                 if (ray_i < 0) continue;
 
                 bool finished = false, fault = false;
-                if (pend_mask == 0) {
-                        // pop until there is work: a world-ray marker restores the
-                        // world ray and pops again in the same step
-                        while ((group.y >> 24) == 0 && sp > 0) {
-                                --sp;
-                                const uint2 e = stack[sp * stride];
-                                if (e.x == 0xFFFFFFFFu) {
-                                        world_ray(rays, ray_i, r);
-                                        set_ray_dirs(r);
-                                        cur_inst = -1;
-                                } else if (e.x & 0x80000000u) {
-                                        pend_base = e.x & 0x7FFFFFFFu;
-                                        pend_mask = e.y;
-                                        break;
+                // leaf records to look at in this step: bits pend_mask of pend_bits
+                uint32_t pend_base = 0, pend_bits = 0, pend_mask = 0;
+                // pop until there is work: a world-ray marker restores the world
+                // ray and pops again in the same step
+                while ((group.y >> 24) == 0 && sp > 0) {
+                        --sp;
+                        const uint2 e = stack[sp * stride];
+                        if (e.x == 0xFFFFFFFFu) {
+                                world_ray(rays, ray_i, r);
+                                set_ray_dirs(r, s.rcp_max);
+                                cur_inst = -1;
+                        } else if (e.x & 0x80000000u) {
+                                pend_base = e.x & 0x7FFFFFFFu;
+                                pend_mask = e.y;
+                                pend_bits = 0xFFFFFFFFu;
+                                break;
+                        } else {
+                                group = e;
+                        }
+                }
+                uint32_t hits = group.y >> 24;
+                if (pend_mask == 0 && hits) {
+                        const uint32_t key = __ffs(hits) - 1;
+                        hits &= hits - 1;
+                        const uint32_t im = group.y & 0xFFu;
+                        const uint32_t slot = key ^ r.oct;
+                        const uint32_t node = group.x + __popc(im & ((1u << slot) - 1u));
+                        if (hits) {
+                                if (sp >= STACK) {
+                                        atomicOr(s.err, kErrStackOverflow);
+                                        fault = true;
                                 } else {
-                                        group = e;
+                                        stack[sp * stride] = make_uint2(group.x, (hits << 24) | im);
+                                        ++sp;
                                 }
                         }
-                        uint32_t hits = group.y >> 24;
-                        if (pend_mask == 0 && hits) {
-                                const uint32_t key = __ffs(hits) - 1;
-                                hits &= hits - 1;
-                                const uint32_t im = group.y & 0xFFu;
-                                const uint32_t slot = key ^ r.oct;
-                                const uint32_t node = group.x + __popc(im & ((1u << slot) - 1u));
-                                if (hits) {
-                                        if (sp >= STACK) {
-                                                atomicOr(s.err, kErrStackOverflow);
-                                                fault = true;
-                                        } else {
-                                                stack[sp * stride] = make_uint2(group.x, (hits << 24) | im);
-                                                ++sp;
-                                        }
-                                }
-                                if (++steps > s.wide_count) {
-                                        atomicOr(s.err, kErrStepCap);
-                                        fault = true;
-                                }
-                                if (!fault) {
-                                        uint32_t nh, nim, cb;
-                                        open_node(s.wide + 5 * (size_t)node, r, thit, nh, nim, cb, pend_mask, pend_base);
-                                        count_lanes(s, 0);
-                                        group = make_uint2(cb, (nh << 24) | nim);
-                                }
+                        if (++steps > s.wide_count) {
+                                atomicOr(s.err, kErrStepCap);
+                                fault = true;
+                        }
+                        if (!fault) {
+                                const NodeHits h = open_node(s.wide + 5 * (size_t)node, r, thit);
+                                count_lanes(s, 0);
+                                group = make_uint2(h.child_base, (h.nodes << 24) | h.imask);
+                                pend_mask = h.tris;
+                                pend_base = h.tri_base;
+                                pend_bits = h.tri_bits;
                         }
                 }
                 while (!fault && pend_mask) {
                         const uint32_t b = __ffs(pend_mask) - 1;
                         pend_mask &= pend_mask - 1;
-                        const uint32_t ti = pend_base + b;
+                        const uint32_t ti = tri_record(pend_base, pend_bits, b);
                         const float4 a = __ldg(s.tv0 + ti);
                         const int tag = __float_as_int(a.w);
                         if (tag < 0) {
@@ -620,9 +629,15 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced(DevScene s, const voi
                                         group.y = 0u;
                                 }
                                 if (pend_mask) {
-                                        stack[sp * stride] = make_uint2(0x80000000u | pend_base, pend_mask);
+                                        // the records left, as plain offsets from pend_base
+                                        uint32_t left = 0;
+                                        while (pend_mask) {
+                                                const uint32_t q = __ffs(pend_mask) - 1;
+                                                pend_mask &= pend_mask - 1;
+                                                left |= 1u << __popc(pend_bits & ((1u << q) - 1u));
+                                        }
+                                        stack[sp * stride] = make_uint2(0x80000000u | pend_base, left);
                                         ++sp;
-                                        pend_mask = 0;
                                 }
                                 stack[sp * stride] = make_uint2(0xFFFFFFFFu, 0u);
                                 ++sp;
@@ -636,7 +651,7 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced(DevScene s, const voi
                                 r.dx = xf_vector(m0, w.dx, w.dy, w.dz);
                                 r.dy = xf_vector(m1, w.dx, w.dy, w.dz);
                                 r.dz = xf_vector(m2, w.dx, w.dy, w.dz);
-                                set_ray_dirs(r);
+                                set_ray_dirs(r, s.rcp_max);
                                 cur_inst = inst;
                                 group = make_uint2((uint32_t)__float_as_int(m3.x), (1u << 24) | (1u << r.oct));
                                 break;

@@ -272,7 +272,10 @@ class Converter {
                         hi = std::max(hi, (double)chi[i]);
                 }
                 const double mag = std::max(std::fabs(lo), std::fabs(hi));
-                double margin = std::ldexp(std::max(mag, hi - lo), -18);
+                // 2^-18 of the coordinates for the rounding of ray and plane
+                // arithmetic, 2^-15 of the extent (under 1 % of a grid step) for
+                // the slab test's folded grid origin (open_node)
+                double margin = std::ldexp(mag, -18) + std::ldexp(hi - lo, -15);
                 if (!(margin > 0)) margin = 1e-30;
                 float p = (float)(lo - margin);
                 while ((double)p > lo - margin) p = std::nextafter(p, -std::numeric_limits<float>::infinity());
@@ -456,7 +459,6 @@ class Converter {
                         // interior children: contiguous, slot order
                         w.child_base = (uint32_t)out->nodes.size();
                         w.tri_base = (uint32_t)out->v0.size();
-                        uint32_t tri_off = 0;
                         for (int s = 0; s < 8; ++s) {
                                 const int k = kid_in_slot[s];
                                 if (k < 0) continue;
@@ -467,7 +469,7 @@ class Converter {
                                         std::vector<int32_t> kids = open_kids(job.kids[k]);
                                         queue.push_back({kids, (uint32_t)out->nodes.size() - 1, job.depth + 1});
                                 } else {
-                                        w.meta[s] = (uint8_t)(0x80u | ((uint32_t)(c.tri_count - 1) << 5) | tri_off);
+                                        w.tri_bits |= ((1u << c.tri_count) - 1u) << (4 * s);
                                         for (int32_t t = 0; t < c.tri_count; ++t) {
                                                 const Tri &tr = tris_[c.tri_first + t];
                                                 float4_ a{tr.p0[0], tr.p0[1], tr.p0[2], 0.0f};
@@ -476,9 +478,9 @@ class Converter {
                                                 out->v1.push_back(float4_{tr.p1[0], tr.p1[1], tr.p1[2], 0.0f});
                                                 out->v2.push_back(float4_{tr.p2[0], tr.p2[1], tr.p2[2], 0.0f});
                                         }
-                                        tri_off += (uint32_t)c.tri_count;
                                 }
                         }
+                        w.imask_perm = wide_imask_perm(w.imask);
                         out->nodes[job.node] = w;
                 }
                 out->depth = depth;
@@ -486,6 +488,12 @@ class Converter {
 };
 
 }  // namespace
+
+float wide_rcp_max(const WideNode *nodes, size_t count) {
+        int e = 0;
+        for (size_t i = 0; i < count; ++i) e = std::max({e, (int)nodes[i].ex, (int)nodes[i].ey, (int)nodes[i].ez});
+        return std::ldexp(1.0f, std::max(40, std::min(64, 127 - 17 - (e - 127))));
+}
 
 gzg_status build_wide_bvh(const gzg_bvh2_node *nodes, int64_t node_count, const gzg_prim_id *prims,
                           int64_t prim_count, const gzg_triangle_mesh *meshes, int64_t mesh_count,
