@@ -284,6 +284,7 @@ LaunchParams params_for(const gzg_scene *s, const gzg_trace_options *o, bool any
         p.n_dev = nullptr;
         p.inst_out = nullptr;
         p.sched = nullptr;
+        p.sched_zeroed = false;
         return p;
 }
 

@@ -21,9 +21,10 @@ struct LaunchParams {
         int32_t *inst_out;             // two-level scenes: hit instance per ray (optional)
         // Persistent launches: the pull counter of the chunk schedule, a
         // device word that no launch running at the same time uses;
-        // launch_trace clears it on the launch's stream first.  Null: the
-        // static schedule.
+        // launch_trace clears it on the launch's stream first unless it is
+        // sched_zeroed.  Null: the static schedule.
         uint32_t *sched;
+        bool sched_zeroed;
 };
 
 // Rays per kernel launch; launch_trace splits larger calls (32-bit chunk

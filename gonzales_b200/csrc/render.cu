@@ -420,10 +420,17 @@ __device__ V3 hg_sample(V3 wo, float g, float u0, float u1, float &value) {
         return v1 * (sin_theta * cosf(phi)) + v2 * (sin_theta * sinf(phi)) + wo * cos_theta;
 }
 
+// Queue counters of one bounce.  A wave has max_depth + 1 such blocks, all
+// cleared by its generate kernel, so no launch between the stages clears or
+// tallies anything (those one-thread kernels and memsets were 25 of the box
+// scene's 45 launches a wave): a stage of bounce b reads and fills block b, its
+// continuations count into block b + 1, and the statistics are summed when the
+// wave ends.
 enum {
-        kCountExt0 = 0, kCountExt1 = 1, kCountShadow = 2, kCountProbe = 3, kCountWaveBase = 4,
-        kCountDielectric = 6, kCountCoated = 7, kCountConductor = 8, kCountCoatedConductor = 9,
-        kCountSched = 10,  // pull counter of the wave's trace launches (one after another on its stream)
+        kCountExt = 0, kCountShadow = 1, kCountProbe = 2,
+        kCountDielectric = 3, kCountCoated = 4, kCountConductor = 5, kCountCoatedConductor = 6,
+        // pull counters of the bounce's three trace launches
+        kCountSchedExt = 7, kCountSchedShadow = 8, kCountSchedProbe = 9,
         kCountWords = 12
 };
 enum { kStatCamera = 0, kStatExt = 1, kStatShadow = 2, kStatProbe = 3, kStatWaves = 4, kStatWords = 8 };
@@ -468,7 +475,9 @@ struct Wave {
         // coated diffuse (from its back), a conductor (from the front of the
         // second half) or a coated conductor (from its back)
         uint32_t *gen_q;
-        uint32_t *counts;      // kCountWords words; wave base as 2 words at kCountWaveBase
+        uint32_t *counts;      // the bounce's kCountWords counters (the wave's first block outside bounces)
+        int32_t count_blocks;  // blocks of the wave: max_depth + 1
+        uint64_t *base;        // first path of the wave
         unsigned long long *stats;  // kStatWords
         // differentiable rendering (single-scene renderers)
         const float *tex;          // texels: count x tex_res x tex_res x 3 (row v, column u)
@@ -512,7 +521,7 @@ __device__ __forceinline__ void store_ray(float4 *q, uint32_t slot, V3 o, float 
 }
 
 __device__ __forceinline__ uint64_t wave_base(const Wave &w) {
-        return (uint64_t)w.counts[kCountWaveBase] | ((uint64_t)w.counts[kCountWaveBase + 1] << 32);
+        return *w.base;
 }
 
 __device__ __forceinline__ uint32_t wave_count(const Wave &w) {
@@ -778,10 +787,13 @@ __global__ void k_generate(Wave w) {
         zs_block_init();
         const uint32_t count = wave_count(w);
         const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-        if (threadIdx.x == 0 && blockIdx.x == 0) {
-                w.counts[kCountExt0] = count;
-                atomicAdd(w.stats + kStatCamera, (unsigned long long)count);
-                atomicAdd(w.stats + kStatWaves, 1ull);
+        if (blockIdx.x == 0) {
+                for (int k = threadIdx.x; k < w.count_blocks * kCountWords; k += blockDim.x)
+                        w.counts[k] = k == kCountExt ? count : 0u;
+                if (threadIdx.x == 0) {
+                        atomicAdd(w.stats + kStatCamera, (unsigned long long)count);
+                        atomicAdd(w.stats + kStatWaves, 1ull);
+                }
         }
         if (i >= count) return;
         const uint64_t path = wave_base(w) + i;
@@ -892,7 +904,7 @@ __device__ __forceinline__ int entry_key(const Wave &w, const DevScene &s, int c
 }
 
 __global__ void k_sort_count(Wave w, DevScene s, int cur) {
-        const uint32_t n = w.counts[cur];
+        const uint32_t n = w.counts[kCountExt];
         const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
         if (i >= n) return;
         atomicAdd(w.key_hist + entry_key(w, s, cur, i), 1u);
@@ -923,7 +935,7 @@ __global__ void k_sort_scan(Wave w) {
 }
 
 __global__ void k_sort_scatter(Wave w, DevScene s, int cur) {
-        const uint32_t n = w.counts[cur];
+        const uint32_t n = w.counts[kCountExt];
         const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
         if (i >= n) return;
         const uint32_t pos = atomicAdd(w.key_hist + w.key_count + entry_key(w, s, cur, i), 1u);
@@ -1064,7 +1076,7 @@ __device__ void shade_generic(const Wave &w, const DevScene &s, const SceneConst
                         }
                         if (alive) {
                                 const int nxt = cur ^ 1;
-                                const uint32_t q = queue_slot(w.counts + nxt);
+                                const uint32_t q = queue_slot(w.counts + kCountWords + kCountExt);
                                 store_ray(w.q_ray[nxt], q, o, kInf, wi, sc.root);
                                 w.q_id[nxt][q] = path;
                         }
@@ -1200,7 +1212,7 @@ __device__ void shade_medium(const Wave &w, const DevScene &s, const SceneConst 
         }
         if (alive) {
                 const int nxt = cur ^ 1;
-                const uint32_t q = queue_slot(w.counts + nxt);
+                const uint32_t q = queue_slot(w.counts + kCountWords + kCountExt);
                 store_ray(w.q_ray[nxt], q, p, kInf, wi, sc.root);
                 w.q_id[nxt][q] = path;
         }
@@ -1236,7 +1248,7 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
                 if (slot >= n) return;
                 i = w.gen_q[gen_pos(w, kKind, slot)];
         } else {
-                const uint32_t n = w.counts[cur];
+                const uint32_t n = w.counts[kCountExt];
                 if (slot >= n) return;
                 i = sorted ? w.order[slot] : slot;
         }
@@ -1505,7 +1517,7 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
                         }
                         if (alive) {
                                 const int nxt = cur ^ 1;
-                                const uint32_t q = queue_slot(w.counts + nxt);
+                                const uint32_t q = queue_slot(w.counts + kCountWords + kCountExt);
                                 store_ray(w.q_ray[nxt], q, o, kInf, wi, sc.root);
                                 w.q_id[nxt][q] = path;
                         }
@@ -1575,22 +1587,18 @@ __global__ void k_probe_resolve(Wave w, DevScene s, int any_only) {
         w.L[path] = L;
 }
 
-// Per-bounce bookkeeping: ray statistics of the bounce.
-__global__ void k_bounce_tally(Wave w, int cur) {
-        atomicAdd(w.stats + kStatExt, (unsigned long long)w.counts[cur]);
-        atomicAdd(w.stats + kStatShadow, (unsigned long long)w.counts[kCountShadow]);
-        atomicAdd(w.stats + kStatProbe, (unsigned long long)w.counts[kCountProbe]);
-}
-
-// Clears the counters of the queues the next stages fill.
-__global__ void k_clear_counts(Wave w, int next) {
-        w.counts[next] = 0;
-        w.counts[kCountShadow] = 0;
-        w.counts[kCountProbe] = 0;
-        w.counts[kCountDielectric] = 0;
-        w.counts[kCountCoated] = 0;
-        w.counts[kCountConductor] = 0;
-        w.counts[kCountCoatedConductor] = 0;
+// Ray statistics of a wave, by one thread after its last bounce.
+__device__ void tally(const Wave &w) {
+        unsigned long long ext = 0, shadow = 0, probe = 0;
+        for (int b = 0; b + 1 < w.count_blocks; ++b) {
+                const uint32_t *c = w.counts + b * kCountWords;
+                ext += c[kCountExt];
+                shadow += c[kCountShadow];
+                probe += c[kCountProbe];
+        }
+        atomicAdd(w.stats + kStatExt, ext);
+        atomicAdd(w.stats + kStatShadow, shadow);
+        atomicAdd(w.stats + kStatProbe, probe);
 }
 
 // Film.add (Core/Film.swift:107-119): the sample's light scaled by iso / 100
@@ -1668,6 +1676,7 @@ __global__ void k_accumulate_f64(Wave w, double *film_rgb, double *film_sq, doub
 __global__ void k_store_total(Wave w) {
         const uint32_t count = wave_count(w);
         const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+        if (i == 0) tally(w);
         if (i >= count) return;
         w.Ltot[i] = w.L[i];
 }
@@ -1690,15 +1699,11 @@ __global__ void k_emission_gradient(Wave w) {
 }
 
 __global__ void k_advance_wave(Wave w) {
-        const uint64_t next = wave_base(w) + wave_count(w);
-        w.counts[kCountWaveBase] = (uint32_t)(next & 0xFFFFFFFFull);
-        w.counts[kCountWaveBase + 1] = (uint32_t)(next >> 32);
+        tally(w);
+        *w.base = wave_base(w) + wave_count(w);
 }
 
-__global__ void k_set_wave_base(Wave w, uint64_t base) {
-        w.counts[kCountWaveBase] = (uint32_t)(base & 0xFFFFFFFFull);
-        w.counts[kCountWaveBase + 1] = (uint32_t)(base >> 32);
-}
+__global__ void k_set_wave_base(Wave w, uint64_t base) { *w.base = base; }
 
 struct KindList {
         int32_t k[64];
@@ -1962,11 +1967,14 @@ struct gzg_renderer {
                         k_generate<<<grid, block, 0, st>>>(w);
                 }
                 int cur = 0;
+                uint32_t *const first_counts = w.counts;
+                Wave w = this->w;  // w.counts moves with the bounce
                 for (int b = 0; b < max_depth; ++b) {
-                        k_clear_counts<<<1, 1, 0, st>>>(w, cur ^ 1);
+                        w.counts = first_counts + (size_t)b * kCountWords;
                         LaunchParams lp = lp_closest, lpa = lp_any;
-                        lp.sched = lpa.sched = w.counts + kCountSched;
-                        lp.n_dev = w.counts + cur;
+                        lp.sched_zeroed = lpa.sched_zeroed = true;
+                        lp.sched = w.counts + kCountSchedExt;
+                        lp.n_dev = w.counts + kCountExt;
                         lp.inst_out = w.hit_inst;
                         NvtxRange extend_range("gzg extend");
                         cudaError_t e = launch_trace(view, lp, kRayDevice, kOutHit, w.q_ray[cur], nullptr, w.capacity,
@@ -1992,12 +2000,14 @@ struct gzg_renderer {
                         shade_range.end();
                         NvtxRange shadow_range("gzg shadow");
                         lpa.n_dev = w.counts + kCountShadow;
+                        lpa.sched = w.counts + kCountSchedShadow;
                         e = launch_trace(view, lpa, kRayDevice, kOutAnyPrim, w.sh_ray, nullptr, w.capacity, w.sh_occ, st);
                         if (e != cudaSuccess) return e;
                         k_shadow_resolve<<<grid, block, 0, st>>>(w);
                         shadow_range.end();
                         NvtxRange probe_range("gzg probe");
                         if (corrected) {
+                                lp.sched = lpa.sched = w.counts + kCountSchedProbe;
                                 if (probe_any) {
                                         lpa.n_dev = w.counts + kCountProbe;
                                         e = launch_trace(view, lpa, kRayDevice, kOutAnyPrim, w.pr_ray, nullptr, w.capacity,
@@ -2011,9 +2021,9 @@ struct gzg_renderer {
                                 if (e != cudaSuccess) return e;
                                 k_probe_resolve<<<grid, block, 0, st>>>(w, view, probe_any ? 1 : 0);
                         }
-                        k_bounce_tally<<<1, 1, 0, st>>>(w, cur);
                         cur ^= 1;
                 }
+                w.counts = first_counts;
                 NvtxRange accumulate_range("gzg accumulate");
                 if (w.mode == kPrimal) {
                         k_store_total<<<grid, block, 0, st>>>(w);  // the replay runs the same paths
@@ -2307,6 +2317,8 @@ gzg_status renderer_create(gzg_scene *const *scenes, const gzg_render_params *pa
             1, std::min<uint64_t>(std::max<uint64_t>(want, kDefaultWave), w.total_paths));
         const size_t C = r->max_capacity;
         w.scene_count = (int32_t)n;
+        w.count_blocks = 1;
+        for (const gzg_render_params &P : r->params) w.count_blocks = std::max(w.count_blocks, (int32_t)P.max_depth + 1);
         const size_t keys = (size_t)std::max<int64_t>(n, r->view.material_count) + 1;
         if (keys > (1u << 20)) return set_error(GZG_ERR_LIMIT, "renderer: more than 2^20 sort keys");
         const SceneConst *scd = nullptr;
@@ -2320,12 +2332,13 @@ gzg_status renderer_create(gzg_scene *const *scenes, const gzg_render_params *pa
             (st = r->alloc(&w.sh_occ, C)) || (st = r->alloc(&w.pr_ray, 2 * C)) || (st = r->alloc(&w.pr_id, C)) ||
             (st = r->alloc(&w.pr_contrib, C)) || (st = r->alloc(&w.pr_hits, C)) || (st = r->alloc(&w.order, C)) || (st = r->alloc(&w.gen_q, 2 * C)) ||
             (st = r->alloc(&w.alb, C)) || (st = r->alloc(&w.nrm, C)) ||
-            (st = r->alloc(&w.key_hist, 2 * keys)) || (st = r->alloc(&w.counts, kCountWords)) ||
-            (st = r->alloc(&w.stats, kStatWords)))
+            (st = r->alloc(&w.key_hist, 2 * keys)) || (st = r->alloc(&w.counts, (size_t)w.count_blocks * kCountWords)) ||
+            (st = r->alloc(&w.base, 1)) || (st = r->alloc(&w.stats, kStatWords)))
                 return st;
         if (r->view.instances && ((st = r->alloc(&w.hit_inst, C)) || (st = r->alloc(&w.pr_inst, C)))) return st;
         if ((st = cuda_err(cudaMemset(w.key_hist, 0, 2 * keys * sizeof(uint32_t)), "sort histogram"))) return st;
-        if ((st = cuda_err(cudaMemset(w.counts, 0, kCountWords * 4), "renderer counters"))) return st;
+        if ((st = cuda_err(cudaMemset(w.counts, 0, (size_t)w.count_blocks * kCountWords * 4), "renderer counters"))) return st;
+        if ((st = cuda_err(cudaMemset(w.base, 0, 8), "renderer counters"))) return st;
         if ((st = cuda_err(cudaMemset(w.stats, 0, kStatWords * 8), "renderer statistics"))) return st;
         r->configure((uint32_t)std::min<uint64_t>(want, w.total_paths), r->opts.sort_key);
         *out = r.release();

@@ -861,7 +861,7 @@ cudaError_t launch_wide_kernel(TraceKernel k, int stack, bool persistent, const 
                                 k<<<(unsigned)grid, block, smem, st>>>(ws, rays, tmax, n, out);
                                 return cudaGetLastError();
                         }
-                        const cudaError_t e = cudaMemsetAsync(s.sched, 0, sizeof(uint32_t), st);
+                        const cudaError_t e = p.sched_zeroed ? cudaSuccess : cudaMemsetAsync(s.sched, 0, sizeof(uint32_t), st);
                         if (e != cudaSuccess) return e;
                 }
         }
