@@ -32,6 +32,11 @@ struct DevScene {
         unsigned long long *counters;  // optional fetch counters (nodes, triangles, rays)
         uint32_t *sched;               // persistent kernels: per-launch pull counter (zero at launch) or null
         const uint32_t *n_dev;         // optional device-side ray count (overrides the launch's n)
+        // kOutShadow launches: per ray its path and contribution, and the
+        // paths' radiance that unoccluded contributions are added to
+        const uint32_t *shadow_path;
+        const float4 *shadow_contrib;
+        float4 *shadow_radiance;
         // shading data (path integrator)
         const float4 *materials;       // 2 x float4 per material: albedo + type, emission
         const float4 *mat_params;      // per material 3 x float4 (gzg_material_params; null: none)
@@ -221,7 +226,9 @@ __device__ __forceinline__ RayIn load_ray(const void *rays, const float *tmax, i
 
 // ------------------------------------------------------------ hit output
 
-enum OutFormat { kOutHit = 0, kOutIntersection = 1, kOutAnyPrim = 2, kOutOccluded = 3 };
+// kOutShadow: no output array; an unoccluded ray adds its contribution to its
+// path's radiance (DevScene::shadow_*; at most one ray of a launch per path).
+enum OutFormat { kOutHit = 0, kOutIntersection = 1, kOutAnyPrim = 2, kOutOccluded = 3, kOutShadow = 4 };
 
 template <int FMT>
 __device__ __forceinline__ void store_hit(const DevScene &s, void *out, int64_t i, int prim, float t, float u, float v) {
@@ -243,6 +250,15 @@ __device__ __forceinline__ void store_hit(const DevScene &s, void *out, int64_t 
                 __stcs(o, w0);
                 __stcs(o + 1, w1);
                 __stcs(o + 2, make_uint4(__float_as_uint(t), __float_as_uint(u), __float_as_uint(v), prim >= 0 ? 1u : 0u));
+        } else if (FMT == kOutShadow) {
+                if (prim >= 0) return;
+                float4 *radiance = s.shadow_radiance + __ldg(s.shadow_path + i);
+                const float4 c = __ldg(s.shadow_contrib + i);
+                float4 L = *radiance;
+                L.x += c.x;
+                L.y += c.y;
+                L.z += c.z;
+                *radiance = L;
         } else if (FMT == kOutAnyPrim) {
                 __stcs(reinterpret_cast<int *>(out) + i, prim);
         } else {

@@ -27,6 +27,14 @@ struct LaunchParams {
         bool sched_zeroed;
 };
 
+// Where a kOutShadow launch finds its rays' paths and contributions and adds
+// the unoccluded ones.
+struct ShadowSink {
+        const uint32_t *path;
+        const float4 *contrib;
+        float4 *radiance;
+};
+
 // Rays per kernel launch; launch_trace splits larger calls (32-bit chunk
 // indices in the persistent kernels).
 constexpr int64_t kMaxLaunchRays = int64_t(1) << 30;
@@ -34,6 +42,11 @@ constexpr int64_t kMaxLaunchRays = int64_t(1) << 30;
 // ray_fmt: RayFormat; out_fmt: OutFormat.  Asynchronous on `st`.
 cudaError_t launch_trace(const DevScene &s, const LaunchParams &p, int ray_fmt, int out_fmt, const void *rays,
                          const float *tmax, int64_t n, void *out, cudaStream_t st);
+
+// Any hit of a renderer's shadow queue (device rays, persistent wide traversal,
+// Moller-Trumbore leaves) whose unoccluded rays add their contributions.
+cudaError_t launch_shadow(const DevScene &s, const LaunchParams &p, const void *rays, int64_t n, const ShadowSink &sink,
+                          cudaStream_t st);
 
 cudaError_t launch_hits_to_isect(const DevScene &s, const void *hits, int64_t n, void *out, cudaStream_t st);
 

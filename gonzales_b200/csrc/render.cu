@@ -12,7 +12,8 @@
 //     shade    emission, light choice + light sample (-> shadow queue),
 //              MIS BSDF sample (-> probe queue, corrected MIS only),
 //              continuation sample, Russian roulette (-> next extension queue)
-//     shadow   any hit of the shadow queue, then add unoccluded contributions
+//     shadow   any hit of the shadow queue; unoccluded rays add their
+//              contributions as they finish
 //     probe    closest hit of the probe queue, then add emission it reaches
 //   accumulate film sums (radiance, its square, filter weight) with atomics
 //
@@ -460,7 +461,6 @@ struct Wave {
         float4 *sh_ray;
         uint32_t *sh_id;
         float4 *sh_contrib;
-        int32_t *sh_occ;
         float4 *pr_ray;
         uint32_t *pr_id;
         float4 *pr_contrib;
@@ -1528,21 +1528,6 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
         w.zs_dim[path] = z.dim;
 }
 
-// Adds unoccluded shadow-ray contributions.
-__global__ void k_shadow_resolve(Wave w) {
-        const uint32_t n = w.counts[kCountShadow];
-        const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-        if (i >= n) return;
-        if (w.sh_occ[i] >= 0) return;
-        const uint32_t path = w.sh_id[i];
-        const float4 c = w.sh_contrib[i];
-        float4 L = w.L[path];
-        L.x += c.x;
-        L.y += c.y;
-        L.z += c.z;
-        w.L[path] = L;
-}
-
 // Adds the radiance a BSDF probe reaches: the emission of an area light whose
 // normal faces back along the probe, or, on a miss, the environment light.
 // any_only: the view has no area light and the probes were traced as any-hit
@@ -2001,9 +1986,8 @@ struct gzg_renderer {
                         NvtxRange shadow_range("gzg shadow");
                         lpa.n_dev = w.counts + kCountShadow;
                         lpa.sched = w.counts + kCountSchedShadow;
-                        e = launch_trace(view, lpa, kRayDevice, kOutAnyPrim, w.sh_ray, nullptr, w.capacity, w.sh_occ, st);
+                        e = launch_shadow(view, lpa, w.sh_ray, w.capacity, ShadowSink{w.sh_id, w.sh_contrib, w.L}, st);
                         if (e != cudaSuccess) return e;
-                        k_shadow_resolve<<<grid, block, 0, st>>>(w);
                         shadow_range.end();
                         NvtxRange probe_range("gzg probe");
                         if (corrected) {
@@ -2329,7 +2313,7 @@ gzg_status renderer_create(gzg_scene *const *scenes, const gzg_render_params *pa
             (st = r->alloc(&w.weight, C)) || (st = r->alloc(&w.q_ray[0], 2 * C)) || (st = r->alloc(&w.q_ray[1], 2 * C)) ||
             (st = r->alloc(&w.q_id[0], C)) || (st = r->alloc(&w.q_id[1], C)) || (st = r->alloc(&w.hits, C)) ||
             (st = r->alloc(&w.sh_ray, 2 * C)) || (st = r->alloc(&w.sh_id, C)) || (st = r->alloc(&w.sh_contrib, C)) ||
-            (st = r->alloc(&w.sh_occ, C)) || (st = r->alloc(&w.pr_ray, 2 * C)) || (st = r->alloc(&w.pr_id, C)) ||
+            (st = r->alloc(&w.pr_ray, 2 * C)) || (st = r->alloc(&w.pr_id, C)) ||
             (st = r->alloc(&w.pr_contrib, C)) || (st = r->alloc(&w.pr_hits, C)) || (st = r->alloc(&w.order, C)) || (st = r->alloc(&w.gen_q, 2 * C)) ||
             (st = r->alloc(&w.alb, C)) || (st = r->alloc(&w.nrm, C)) ||
             (st = r->alloc(&w.key_hist, 2 * keys)) || (st = r->alloc(&w.counts, (size_t)w.count_blocks * kCountWords)) ||

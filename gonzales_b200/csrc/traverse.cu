@@ -942,7 +942,8 @@ cudaError_t launch_trace(const DevScene &scene, const LaunchParams &p, int ray_f
         s.sched = p.sched;
         if (s.instances) {
                 // two-level scenes: persistent wide traversal only
-                if (ray_fmt != kRayDevice || (out_fmt != kOutHit && out_fmt != kOutAnyPrim)) return cudaErrorNotSupported;
+                if (ray_fmt != kRayDevice || (out_fmt != kOutHit && out_fmt != kOutAnyPrim && out_fmt != kOutShadow))
+                        return cudaErrorNotSupported;
                 const int need = p.wide_depth > 1 ? p.wide_depth : 1;
                 const int want = p.stack_depth > need ? p.stack_depth : need;
                 LaunchParams q = p;
@@ -951,15 +952,33 @@ cudaError_t launch_trace(const DevScene &scene, const LaunchParams &p, int ray_f
                 int stack;
                 if (want <= 16) {
                         stack = 16;
-                        k = out_fmt == kOutHit ? k_wide_instanced<kOutHit, false, 16> : k_wide_instanced<kOutAnyPrim, true, 16>;
+                        k = out_fmt == kOutHit ? k_wide_instanced<kOutHit, false, 16>
+                            : out_fmt == kOutShadow ? k_wide_instanced<kOutShadow, true, 16>
+                                                    : k_wide_instanced<kOutAnyPrim, true, 16>;
                 } else if (want <= 32) {
                         stack = 32;
-                        k = out_fmt == kOutHit ? k_wide_instanced<kOutHit, false, 32> : k_wide_instanced<kOutAnyPrim, true, 32>;
+                        k = out_fmt == kOutHit ? k_wide_instanced<kOutHit, false, 32>
+                            : out_fmt == kOutShadow ? k_wide_instanced<kOutShadow, true, 32>
+                                                    : k_wide_instanced<kOutAnyPrim, true, 32>;
                 } else {
                         stack = 64;
-                        k = out_fmt == kOutHit ? k_wide_instanced<kOutHit, false, 64> : k_wide_instanced<kOutAnyPrim, true, 64>;
+                        k = out_fmt == kOutHit ? k_wide_instanced<kOutHit, false, 64>
+                            : out_fmt == kOutShadow ? k_wide_instanced<kOutShadow, true, 64>
+                                                    : k_wide_instanced<kOutAnyPrim, true, 64>;
                 }
                 return launch_wide_kernel(k, stack, true, q, s, rays, tmax, n, out, st);
+        }
+        if (out_fmt == kOutShadow) {
+                // a renderer's shadow queue: one traversal, one leaf test
+                if (ray_fmt != kRayDevice) return cudaErrorNotSupported;
+                const int need = p.wide_depth > 2 ? p.wide_depth - 1 : 1;
+                const int want = p.stack_depth > need ? p.stack_depth : need;
+                const TraceKernel k = want <= 8    ? k_wide_persistent<kRayDevice, kOutShadow, true, 8, GZG_LEAF_MOLLER_TRUMBORE>
+                                      : want <= 16 ? k_wide_persistent<kRayDevice, kOutShadow, true, 16, GZG_LEAF_MOLLER_TRUMBORE>
+                                      : want <= 32 ? k_wide_persistent<kRayDevice, kOutShadow, true, 32, GZG_LEAF_MOLLER_TRUMBORE>
+                                                   : k_wide_persistent<kRayDevice, kOutShadow, true, 64, GZG_LEAF_MOLLER_TRUMBORE>;
+                const int stack = want <= 8 ? 8 : want <= 16 ? 16 : want <= 32 ? 32 : 64;
+                return launch_wide_kernel(k, stack, true, p, s, rays, tmax, n, out, st);
         }
         if (ray_fmt == kRayDevice) {
                 switch (out_fmt) {
@@ -975,6 +994,16 @@ cudaError_t launch_trace(const DevScene &scene, const LaunchParams &p, int ray_f
         case kOutAnyPrim: return launch_fmt<kRayReference, kOutAnyPrim, true>(s, p, rays, tmax, n, out, st);
         default: return launch_fmt<kRayReference, kOutOccluded, true>(s, p, rays, tmax, n, out, st);
         }
+}
+
+cudaError_t launch_shadow(const DevScene &scene, const LaunchParams &p, const void *rays, int64_t n,
+                          const ShadowSink &sink, cudaStream_t st) {
+        if (n > kMaxLaunchRays) return cudaErrorInvalidValue;
+        DevScene s = scene;
+        s.shadow_path = sink.path;
+        s.shadow_contrib = sink.contrib;
+        s.shadow_radiance = sink.radiance;
+        return launch_trace(s, p, kRayDevice, kOutShadow, rays, nullptr, n, nullptr, st);
 }
 
 cudaError_t launch_hits_to_isect(const DevScene &s, const void *hits, int64_t n, void *out, cudaStream_t st) {
