@@ -494,7 +494,8 @@ struct Wave {
         // two-level scenes: the instance of each extension and probe hit
         int32_t *hit_inst;
         int32_t *pr_inst;
-        // first-hit AOVs per path slot: BSDF albedo and geometric normal
+        // first-hit AOVs per path slot: BSDF albedo and geometric normal (null
+        // in a pass without AOV films)
         float4 *alb;
         float4 *nrm;
 };
@@ -522,6 +523,12 @@ __device__ __forceinline__ void store_ray(float4 *q, uint32_t slot, V3 o, float 
 
 __device__ __forceinline__ uint64_t wave_base(const Wave &w) {
         return *w.base;
+}
+
+// The scene of a path.  One-scene renderers keep no index per path: reading it
+// would put a dependent load before every use of the scene's constants.
+__device__ __forceinline__ const SceneConst &path_scene(const Wave &w, uint32_t path) {
+        return w.scenes[w.scene_count == 1 ? 0u : w.scene[path]];
 }
 
 __device__ __forceinline__ uint32_t wave_count(const Wave &w) {
@@ -807,8 +814,8 @@ __global__ void k_generate(Wave w) {
         }
         const SceneConst &sc = w.scenes[lo];
         const uint64_t q = path - sc.path_begin;
-        const uint32_t pixel = (uint32_t)(q / (uint64_t)sc.spp);
-        const uint32_t sample = (uint32_t)(q % (uint64_t)sc.spp) + (uint32_t)sc.first_sample;
+        const uint32_t pixel = (q >> 32) == 0 ? (uint32_t)q / (uint32_t)sc.spp : (uint32_t)(q / (uint64_t)sc.spp);
+        const uint32_t sample = (uint32_t)(q - (uint64_t)pixel * (uint32_t)sc.spp) + (uint32_t)sc.first_sample;
         const uint32_t px = (uint32_t)sc.crop_x0 + pixel % (uint32_t)sc.crop_w,
                        py = (uint32_t)sc.crop_y0 + pixel / (uint32_t)sc.crop_w;
         ZSobol z;
@@ -819,10 +826,12 @@ __global__ void k_generate(Wave w) {
         w.zs_dim[i] = z.dim;
         w.thr[i] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
         w.L[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        w.alb[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        w.nrm[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (w.alb) {
+                w.alb[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                w.nrm[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
         w.pixel[i] = sc.film_offset + pixel;
-        w.scene[i] = (uint32_t)lo;
+        if (w.scene_count > 1) w.scene[i] = (uint32_t)lo;
         w.weight[i] = weight;
         store_ray(w.q_ray[0], i, org, kInf, dir, sc.root);
         w.q_id[0][i] = i;
@@ -890,7 +899,7 @@ __device__ __forceinline__ V3 offset_origin(V3 p, V3 n, V3 dir) {
 __device__ __forceinline__ int entry_key(const Wave &w, const DevScene &s, int cur, uint32_t i) {
         const int prim = __float_as_int(w.hits[i].w);
         if (prim < 0) return w.key_count - 1;
-        if (w.sort_key == kSortScene) return (int)w.scene[w.q_id[cur][i]];
+        if (w.sort_key == kSortScene) return w.scene_count == 1 ? 0 : (int)w.scene[w.q_id[cur][i]];
         int gp = prim;
         if (s.instances) {
                 const float4 w3 = __ldg(s.instances + 4 * w.hit_inst[i] + 3);
@@ -899,7 +908,7 @@ __device__ __forceinline__ int entry_key(const Wave &w, const DevScene &s, int c
         int type;
         int64_t m;
         prim_info(s, gp, type, m);
-        if (type == 3) m = w.scenes[w.scene[w.q_id[cur][i]]].material_begin;
+        if (type == 3) m = path_scene(w, w.q_id[cur][i]).material_begin;
         return m >= 0 && m < w.key_count - 1 ? (int)m : w.key_count - 1;
 }
 
@@ -1258,7 +1267,7 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
         const float4 rd = w.q_ray[cur][2 * i + 1];
         const V3 d = v3(rd);
         if (kKind < kShadeDielectric) {
-                const SceneConst &scm = w.scenes[w.scene[path]];
+                const SceneConst &scm = path_scene(w, path);
                 if (scm.has_medium) {
                         // Homogeneous.sample on the segment before it is shaded (the
                         // branch of shadeBounce :394-408 as meant to run); its two
@@ -1302,7 +1311,7 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
                 }
                 return;
         }
-        const SceneConst &sc = w.scenes[w.scene[path]];
+        const SceneConst &sc = path_scene(w, path);
         const float4 t4 = w.thr[path];
         V3 thr = v3(t4);
         const bool after_specular = t4.w != 0.0f;
@@ -1333,7 +1342,7 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
                 }
                 if (kKind >= kShadeDielectric) {
                         const V3 base = v3(m0);
-                        if (bounce == 0) {
+                        if (bounce == 0 && w.alb) {
                                 // Bsdf.albedo(): the base reflectance of a coated diffuse,
                                 // white for the dielectric and the conductors
                                 const V3 a = kKind == kShadeCoated ? base : v3(1.0f, 1.0f, 1.0f);
@@ -1371,7 +1380,7 @@ __global__ void __launch_bounds__(128, kKind == kShadeSplit                     
                 }
         }
         const V3 f_val = refl * (1.0f / kPi);
-        if (bounce == 0) {
+        if (bounce == 0 && w.alb) {
                 // surfaceEstimate (:341-344): state.albedo, state.firstNormal
                 w.alb[path] = make_float4(refl.x, refl.y, refl.z, 0.0f);
                 w.nrm[path] = make_float4(ng.x, ng.y, ng.z, 0.0f);
@@ -1552,12 +1561,12 @@ __global__ void k_probe_resolve(Wave w, DevScene s, int any_only) {
                 int64_t mat_index;
                 prim_info(s, sf.gprim, type, mat_index);
                 if (type != 3 || mat_index < 0 || mat_index >= s.material_count) return;
-                if (!w.scenes[w.scene[w.pr_id[i]]].two_sided && !(dot(sf.ng, neg(wi)) > 0.0f)) return;
+                if (!path_scene(w, w.pr_id[i]).two_sided && !(dot(sf.ng, neg(wi)) > 0.0f)) return;
                 le = v3(__ldg(s.materials + 2 * mat_index + 1)) * w.emission_scale;
         }
         const uint32_t path = w.pr_id[i];
         float4 c = w.pr_contrib[i];
-        const SceneConst &sc = w.scenes[w.scene[path]];
+        const SceneConst &sc = path_scene(w, path);
         if (sc.has_medium) {
                 // the medium's transmittance up to what the probe reaches
                 const V3 tr = medium_tr(sc, v3(w.pr_ray[2 * i]), wi, prim < 0 ? kInf : h.x);
@@ -1589,7 +1598,7 @@ __device__ void tally(const Wave &w) {
 // Film.add (Core/Film.swift:107-119): the sample's light scaled by iso / 100
 // and, when a clamp is set, by max / its largest component.
 __device__ __forceinline__ float4 film_light(const Wave &w, uint32_t i) {
-        const SceneConst &sc = w.scenes[w.scene[i]];
+        const SceneConst &sc = path_scene(w, i);
         float4 L = w.L[i];
         L.x *= sc.film_scale;
         L.y *= sc.film_scale;
@@ -1606,36 +1615,61 @@ __device__ __forceinline__ float4 film_light(const Wave &w, uint32_t i) {
         return L;
 }
 
+// Sums of N values over each run of lanes with the same pixel (a wave's slots
+// are in path order, so a pixel's samples are neighbours); the first lane of a
+// run gets its sum.  same: bit k set when the lane 2^k above is in the run.
+template <int N>
+__device__ __forceinline__ void run_sums(float (&v)[N], unsigned same) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                        const float t = __shfl_down_sync(0xFFFFFFFFu, v[j], 1u << k);
+                        if ((same >> k) & 1u) v[j] += t;
+                }
+}
+
 // Film sums: radiance, its square, the filter weight and the first-hit AOVs
-// (albedo, normal: Tile.swift:157-205), per pixel of the batch film.
+// (albedo, normal: Tile.swift:157-205), per pixel of the batch film.  A warp
+// adds its samples of a pixel together first: the kernel waits on the atomics
+// (16 to one address at 16 spp), not on the 24 bytes it reads per path.
 __global__ void k_accumulate(Wave w, float *film_rgb, float *film_sq, float *film_w, float *film_alb,
                              float *film_nrm) {
         const uint32_t count = wave_count(w);
         const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-        if (i >= count) return;
-        const uint32_t px = w.pixel[i];
-        const float4 L = film_light(w, i);
-        atomicAdd(film_rgb + 3 * (size_t)px, L.x);
-        atomicAdd(film_rgb + 3 * (size_t)px + 1, L.y);
-        atomicAdd(film_rgb + 3 * (size_t)px + 2, L.z);
-        if (film_sq) {
-                atomicAdd(film_sq + 3 * (size_t)px, L.x * L.x);
-                atomicAdd(film_sq + 3 * (size_t)px + 1, L.y * L.y);
-                atomicAdd(film_sq + 3 * (size_t)px + 2, L.z * L.z);
+        const unsigned lane = threadIdx.x & 31u;
+        const uint32_t px = i < count ? w.pixel[i] : 0xFFFFFFFFu;  // below 2^32 - 1 pixels
+        unsigned same = 0u;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+                const uint32_t above = __shfl_down_sync(0xFFFFFFFFu, px, 1u << k);
+                if (lane + (1u << k) < 32u && above == px) same |= 1u << k;
         }
-        atomicAdd(film_w + px, w.weight[i]);
-        if (film_alb) {
-                const float4 a = w.alb[i];
-                atomicAdd(film_alb + 3 * (size_t)px, a.x);
-                atomicAdd(film_alb + 3 * (size_t)px + 1, a.y);
-                atomicAdd(film_alb + 3 * (size_t)px + 2, a.z);
+        const uint32_t below = __shfl_up_sync(0xFFFFFFFFu, px, 1u);
+        const bool first = i < count && (lane == 0u || below != px);
+        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 L = i < count ? film_light(w, i) : zero;
+        const size_t p3 = 3 * (size_t)px;
+        float v[4] = {L.x, L.y, L.z, i < count ? w.weight[i] : 0.0f};
+        run_sums(v, same);
+        if (first) {
+                atomicAdd(film_rgb + p3, v[0]);
+                atomicAdd(film_rgb + p3 + 1, v[1]);
+                atomicAdd(film_rgb + p3 + 2, v[2]);
+                atomicAdd(film_w + px, v[3]);
         }
-        if (film_nrm) {
-                const float4 nv = w.nrm[i];
-                atomicAdd(film_nrm + 3 * (size_t)px, nv.x);
-                atomicAdd(film_nrm + 3 * (size_t)px + 1, nv.y);
-                atomicAdd(film_nrm + 3 * (size_t)px + 2, nv.z);
-        }
+        auto add = [&](float *film, float4 a) {
+                float u[3] = {a.x, a.y, a.z};
+                run_sums(u, same);
+                if (first) {
+                        atomicAdd(film + p3, u[0]);
+                        atomicAdd(film + p3 + 1, u[1]);
+                        atomicAdd(film + p3 + 2, u[2]);
+                }
+        };
+        if (film_sq) add(film_sq, make_float4(L.x * L.x, L.y * L.y, L.z * L.z, 0.0f));
+        if (film_alb) add(film_alb, i < count ? w.alb[i] : zero);
+        if (film_nrm) add(film_nrm, i < count ? w.nrm[i] : zero);
 }
 
 // Double-precision film sums (finite differences need sums whose rounding
@@ -1928,6 +1962,8 @@ struct gzg_renderer {
         // One wave: generate, bounces, then by w.mode accumulate + advance,
         // keep the primal radiance, or finish a replay + advance.  Enqueued on st.
         cudaError_t enqueue_wave(const Films &film, cudaStream_t st) {
+                Wave w = this->w;  // w.counts moves with the bounce
+                if (!film.alb && !film.nrm) w.alb = w.nrm = nullptr;
                 const int block = 128;
                 const unsigned grid = (w.capacity + block - 1) / block;
                 int max_depth = 0;
@@ -1953,7 +1989,6 @@ struct gzg_renderer {
                 }
                 int cur = 0;
                 uint32_t *const first_counts = w.counts;
-                Wave w = this->w;  // w.counts moves with the bounce
                 for (int b = 0; b < max_depth; ++b) {
                         w.counts = first_counts + (size_t)b * kCountWords;
                         LaunchParams lp = lp_closest, lpa = lp_any;
