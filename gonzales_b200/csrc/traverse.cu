@@ -83,8 +83,15 @@ __device__ __forceinline__ bool chunk_next(ChunkCursor &c, uint32_t *sched, uint
 // slab test compare float bits as integers (below).  A plane then appears at
 // distance |dx| * limit instead of beyond it, still far past any hit distance
 // of a scene with coordinates below about 1e12, so the test stays conservative.
+// The approximate reciprocal is within an ulp; the far planes' slack covers it
+// (an IEEE division costs ten instructions and a branch for each of the three
+// components, at every ray and, on two levels, at every instance entered and
+// left: 8M camera rays 992 -> 919 us, 8M incoherent rays 2,251 -> 2,117, 4M
+// any-hit rays 915 -> 892, 2M rays through 4096 instances 1,380 -> 1,358).
 __device__ __forceinline__ float wide_rcp(float d, float limit) {
-        return copysignf(fminf(fabsf(__fdiv_rn(1.0f, d)), limit), d);
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+        return copysignf(fminf(fabsf(r), limit), d);
 }
 
 // Packed FP32 pairs (sm_100a f32x2): each element rounds exactly as the
@@ -163,8 +170,11 @@ __device__ __forceinline__ NodeHits open_node(const uint4 *__restrict__ node, co
         const float az = (pz - r.oz) * r.rdz;
         // Far planes carry a relative slack (the reference's tFar has 1.0000003,
         // kernel.mojo:204) in their per-node constants instead of one multiply
-        // per child; thit is scaled the same way once.
-        const float kSlack = 1.0000006f;
+        // per child; thit is scaled the same way once.  A plane's distance is
+        // off by at most 3.5 x 2^-23 of itself (reciprocal 1, difference 0.5,
+        // product 0.5, folded constant 1, fma 0.5), a near and a far plane
+        // together by 7; the slack is 9.
+        const float kSlack = 1.0000011f;
         const float fsx = sx * kSlack, fsy = sy * kSlack, fsz = sz * kSlack;
         const float fax = ax * kSlack, fay = ay * kSlack, faz = az * kSlack;
         const int thit_far = __float_as_int(thit * kSlack);
