@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <array>
 #include <cmath>
 #include <cstring>
@@ -62,30 +63,74 @@ class DeviceGuard {
         int prev_ = 0, dev_ = 0;
 };
 
-constexpr int kSlots = 4;
-constexpr int64_t kChunk = 1 << 19;  // rays per pipelined chunk (512K x 4 streams: 2 % faster end to end than 1M x 3)
+constexpr int kSlots = 8;             // chunks in flight of one staged call
+constexpr int kDirectSlots = 4;       // of one that copies from and to pinned host arrays
+constexpr int64_t kChunk = 1 << 19;   // rays per chunk of pinned arrays (512K x 4 streams: 2 % faster end to end than 1M x 3)
+// Staged chunks are small, so that the copies in, the transfers, the trace and
+// the copies out of one call overlap, but no smaller than what a copy's and a
+// launch's overhead is worth.
+constexpr int64_t kStagedChunkMin = 1 << 14, kStagedChunkMax = 1 << 17;
 
-// Per-call staging: device buffers and pinned host buffers for kSlots chunks
-// in flight, each slot with its own stream and its pull counter for the
-// persistent kernel.
+// Per-call staging: device buffers, and pinned host buffers for pageable
+// callers, for kSlots chunks in flight, each slot with its own stream and its
+// pull counter for the persistent kernel.  A slot's buffers are made when a
+// call first needs them and grow to the largest chunk seen.
 struct Staging {
-        cudaStream_t st[kSlots] = {};
-        void *d_in[kSlots] = {}, *d_tmax[kSlots] = {}, *d_out[kSlots] = {};
-        void *h_in[kSlots] = {}, *h_tmax[kSlots] = {}, *h_out[kSlots] = {};
+        struct Slot {
+                cudaStream_t st = nullptr;
+                void *d_in = nullptr, *d_tmax = nullptr, *d_out = nullptr;
+                void *h_in = nullptr, *h_tmax = nullptr, *h_out = nullptr;
+                int64_t d_rays = 0, h_rays = 0;
+        };
+        Slot slot[kSlots];
         uint32_t *d_sched = nullptr;  // one word per slot
         ~Staging() {
                 cudaFree(d_sched);
-                for (int k = 0; k < kSlots; ++k) {
-                        if (st[k]) cudaStreamDestroy(st[k]);
-                        cudaFree(d_in[k]);
-                        cudaFree(d_tmax[k]);
-                        cudaFree(d_out[k]);
-                        cudaFreeHost(h_in[k]);
-                        cudaFreeHost(h_tmax[k]);
-                        cudaFreeHost(h_out[k]);
+                for (Slot &q : slot) {
+                        if (q.st) cudaStreamDestroy(q.st);
+                        free_device(q);
+                        free_host(q);
                 }
         }
+        static void free_device(Slot &q) {
+                cudaFree(q.d_in);
+                cudaFree(q.d_tmax);
+                cudaFree(q.d_out);
+                q.d_in = q.d_tmax = q.d_out = nullptr;
+                q.d_rays = 0;
+        }
+        static void free_host(Slot &q) {
+                cudaFreeHost(q.h_in);
+                cudaFreeHost(q.h_tmax);
+                cudaFreeHost(q.h_out);
+                q.h_in = q.h_tmax = q.h_out = nullptr;
+                q.h_rays = 0;
+        }
+        // Makes slot k ready for chunks of `rays` rays (nothing of it is in flight).
+        gzg_status ensure(int k, int64_t rays, bool host) {
+                Slot &q = slot[k];
+                if (!q.st) GZG_CK(cudaStreamCreateWithFlags(&q.st, cudaStreamNonBlocking), "staging stream");
+                if (q.d_rays < rays) {
+                        free_device(q);
+                        GZG_CK(cudaMalloc(&q.d_in, rays * sizeof(gzg_ray)), "staging device buffer");
+                        GZG_CK(cudaMalloc(&q.d_tmax, rays * sizeof(float)), "staging device buffer");
+                        GZG_CK(cudaMalloc(&q.d_out, rays * sizeof(gzg_intersection)), "staging device buffer");
+                        q.d_rays = rays;
+                }
+                if (host && q.h_rays < rays) {
+                        free_host(q);
+                        GZG_CK(cudaHostAlloc(&q.h_in, rays * sizeof(gzg_ray), cudaHostAllocDefault), "pinned buffer");
+                        GZG_CK(cudaHostAlloc(&q.h_tmax, rays * sizeof(float), cudaHostAllocDefault), "pinned buffer");
+                        GZG_CK(cudaHostAlloc(&q.h_out, rays * sizeof(gzg_intersection), cudaHostAllocDefault), "pinned buffer");
+                        q.h_rays = rays;
+                }
+                return GZG_OK;
+        }
 };
+
+// Helper threads of staged calls running now, over all scenes and callers:
+// callers that already keep every core busy get none.
+std::atomic<int> g_helpers{0};
 
 bool is_pinned(const void *p) {
         cudaPointerAttributes a;
@@ -201,16 +246,6 @@ struct gzg_scene {
                 }
                 auto s = std::make_unique<Staging>();
                 GZG_CK(cudaMalloc(&s->d_sched, kSlots * sizeof(uint32_t)), "staging schedule words");
-                for (int k = 0; k < kSlots; ++k) {
-                        GZG_CK(cudaStreamCreateWithFlags(&s->st[k], cudaStreamNonBlocking), "staging stream");
-                        GZG_CK(cudaMalloc(&s->d_in[k], kChunk * sizeof(gzg_ray_d)), "staging device buffer");
-                        GZG_CK(cudaMalloc(&s->d_tmax[k], kChunk * sizeof(float)), "staging device buffer");
-                        GZG_CK(cudaMalloc(&s->d_out[k], kChunk * sizeof(gzg_intersection)), "staging device buffer");
-                        GZG_CK(cudaHostAlloc(&s->h_in[k], kChunk * sizeof(gzg_ray), cudaHostAllocDefault), "pinned buffer");
-                        GZG_CK(cudaHostAlloc(&s->h_tmax[k], kChunk * sizeof(float), cudaHostAllocDefault), "pinned buffer");
-                        GZG_CK(cudaHostAlloc(&s->h_out[k], kChunk * sizeof(gzg_intersection), cudaHostAllocDefault),
-                               "pinned buffer");
-                }
                 *out = std::move(s);
                 return GZG_OK;
         }
@@ -337,8 +372,12 @@ cudaError_t device_trace(gzg_scene *scene, LaunchParams p, int out_fmt, const vo
         return cudaEventRecord(r.ev[k], st);
 }
 
-// Host batch: chunks of Ray_C + tMax through kSlots streams; results are
-// `out_bytes` per ray in format `out_fmt`.
+// Host batch: chunks of Ray_C + tMax through the slots' streams; results are
+// `out_bytes` per ray in format `out_fmt`.  Pinned arrays are copied from and to
+// directly.  Pageable ones go through the pinned staging buffers, and there the
+// host's copies are what the call waits for (76 bytes a ray through one core:
+// 1M rays took 9.0 ms, of which 1.4 ms PCIe and 0.3 ms tracing), so several
+// threads each take chunks through a slot of their own.
 gzg_status host_batch(gzg_scene *s, const gzg_ray *rays, const float *tmax, int64_t count, void *results,
                       size_t out_bytes, int out_fmt, const gzg_trace_options *opt) {
         if (!s || count < 0 || (count > 0 && (!rays || !tmax || !results)))
@@ -353,61 +392,99 @@ gzg_status host_batch(gzg_scene *s, const gzg_ray *rays, const float *tmax, int6
         std::unique_ptr<Staging> stg;
         st = s->acquire(&stg);
         if (st != GZG_OK) return st;
-        LaunchParams p = params_for(s, opt, out_fmt == kOutAnyPrim || out_fmt == kOutOccluded);
+        const LaunchParams base = params_for(s, opt, out_fmt == kOutAnyPrim || out_fmt == kOutOccluded);
         const bool direct = is_pinned(rays) && is_pinned(tmax) && is_pinned(results);
-        const int64_t nchunks = (count + kChunk - 1) / kChunk;
+        int64_t chunk = kChunk;
+        if (!direct) {
+                // two chunks a slot or more, a power of two so that slots keep few sizes
+                chunk = kStagedChunkMin;
+                while (chunk < kStagedChunkMax && chunk * 2 * kSlots < count) chunk *= 2;
+        }
+        const int64_t nchunks = (count + chunk - 1) / chunk;
+        const int slots = (int)std::min<int64_t>(direct ? kDirectSlots : kSlots, nchunks);
         char *res = reinterpret_cast<char *>(results);
-        // A wait that ran out leaves chunks in flight on the staging streams:
-        // their buffers are left to them (never freed nor pooled again).
-        auto abandon = [&](gzg_status s) -> gzg_status {
-                if (s == GZG_ERR_TIMEOUT) stg.release();
-                return s;
-        };
-        auto drain = [&](int64_t c) -> gzg_status {
-                const int k = (int)(c % kSlots);
-                const gzg_status ws = wait_stream(stg->st[k], "batch chunk");
-                if (ws != GZG_OK) return ws;
-                const int64_t off = c * kChunk, n = std::min(kChunk, count - off);
-                std::memcpy(res + off * out_bytes, stg->h_out[k], (size_t)n * out_bytes);
+        auto enqueue = [&](int k, int64_t c) -> gzg_status {
+                Staging::Slot &q = stg->slot[k];
+                const int64_t off = c * chunk, n = std::min(chunk, count - off);
+                GZG_CK(cudaMemcpyAsync(q.d_in, direct ? (const void *)(rays + off) : q.h_in, (size_t)n * sizeof(gzg_ray),
+                                       cudaMemcpyHostToDevice, q.st),
+                       "ray upload");
+                GZG_CK(cudaMemcpyAsync(q.d_tmax, direct ? (const void *)(tmax + off) : q.h_tmax, (size_t)n * sizeof(float),
+                                       cudaMemcpyHostToDevice, q.st),
+                       "tMax upload");
+                LaunchParams p = base;
+                p.sched = stg->d_sched + k;  // this slot's stream orders its launches
+                GZG_CK(launch_trace(s->dev, p, kRayReference, out_fmt, q.d_in, reinterpret_cast<const float *>(q.d_tmax), n,
+                                    q.d_out, q.st),
+                       "trace launch");
+                GZG_CK(cudaMemcpyAsync(direct ? (void *)(res + off * out_bytes) : q.h_out, q.d_out, (size_t)n * out_bytes,
+                                       cudaMemcpyDeviceToHost, q.st),
+                       "result download");
                 return GZG_OK;
         };
-        for (int64_t c = 0; c < nchunks; ++c) {
-                const int k = (int)(c % kSlots);
-                const int64_t off = c * kChunk, n = std::min(kChunk, count - off);
-                cudaStream_t stream = stg->st[k];
-                const void *src_rays = rays + off;
-                const void *src_tmax = tmax + off;
-                if (!direct) {
-                        if (c >= kSlots) {
-                                st = drain(c - kSlots);
-                                if (st != GZG_OK) return abandon(st);
+        if (direct) {
+                for (int k = 0; k < slots && !st; ++k) st = stg->ensure(k, chunk, false);
+                for (int64_t c = 0; c < nchunks && !st; ++c) st = enqueue((int)(c % slots), c);
+                for (int k = 0; k < slots && !st; ++k) st = wait_stream(stg->slot[k].st, "batch sync");
+        } else {
+                std::atomic<int64_t> next{0};
+                std::atomic<bool> stop{false};
+                gzg_status status[kSlots] = {};
+                std::string message[kSlots];
+                auto work = [&](int k) {
+                        gzg_status ws = GZG_OK;
+                        try {
+                                DeviceGuard tg(s->device);
+                                if (!ws) ws = stg->ensure(k, chunk, true);
+                                Staging::Slot &q = stg->slot[k];
+                                for (int64_t c; !ws && !stop && (c = next.fetch_add(1)) < nchunks;) {
+                                        const int64_t off = c * chunk, n = std::min(chunk, count - off);
+                                        std::memcpy(q.h_in, rays + off, (size_t)n * sizeof(gzg_ray));
+                                        std::memcpy(q.h_tmax, tmax + off, (size_t)n * sizeof(float));
+                                        ws = enqueue(k, c);
+                                        if (!ws) ws = wait_stream(q.st, "batch chunk");
+                                        if (!ws) std::memcpy(res + off * out_bytes, q.h_out, (size_t)n * out_bytes);
+                                }
+                                if (ws) message[k] = g_last_error;
+                        } catch (const std::exception &) {
+                                ws = GZG_ERR_OUT_OF_MEMORY;
                         }
-                        std::memcpy(stg->h_in[k], rays + off, (size_t)n * sizeof(gzg_ray));
-                        std::memcpy(stg->h_tmax[k], tmax + off, (size_t)n * sizeof(float));
-                        src_rays = stg->h_in[k];
-                        src_tmax = stg->h_tmax[k];
+                        if (ws) stop = true;
+                        status[k] = ws;
+                };
+                // helpers beside the calling thread, as far as the cores go
+                int helpers = 0;
+                std::thread helper[kSlots];
+                const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
+                while (helpers + 1 < slots) {
+                        if (g_helpers.fetch_add(1) + 1 >= cores) {
+                                g_helpers.fetch_sub(1);
+                                break;
+                        }
+                        try {
+                                helper[helpers] = std::thread(work, helpers + 1);
+                        } catch (const std::exception &) {
+                                g_helpers.fetch_sub(1);
+                                break;
+                        }
+                        ++helpers;
                 }
-                GZG_CK(cudaMemcpyAsync(stg->d_in[k], src_rays, (size_t)n * sizeof(gzg_ray), cudaMemcpyHostToDevice, stream),
-                       "ray upload");
-                GZG_CK(cudaMemcpyAsync(stg->d_tmax[k], src_tmax, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, stream),
-                       "tMax upload");
-                p.sched = stg->d_sched + k;  // this slot's stream orders its launches
-                GZG_CK(launch_trace(s->dev, p, kRayReference, out_fmt, stg->d_in[k],
-                                    reinterpret_cast<const float *>(stg->d_tmax[k]), n, stg->d_out[k], stream),
-                       "trace launch");
-                void *dst = direct ? (void *)(res + off * out_bytes) : stg->h_out[k];
-                GZG_CK(cudaMemcpyAsync(dst, stg->d_out[k], (size_t)n * out_bytes, cudaMemcpyDeviceToHost, stream),
-                       "result download");
+                work(0);
+                for (int k = 0; k < helpers; ++k) helper[k].join();
+                g_helpers.fetch_sub(helpers);
+                // a wait that ran out comes before any other failure: its
+                // chunk is still in flight
+                for (int pass = 0; pass < 2 && !st; ++pass)
+                        for (int k = 0; k <= helpers && !st; ++k)
+                                if (status[k] && (pass == 1 || status[k] == GZG_ERR_TIMEOUT))
+                                        st = set_error(status[k], message[k].empty() ? "batch call: out of host memory" : message[k]);
         }
-        if (!direct) {
-                for (int64_t c = std::max<int64_t>(0, nchunks - kSlots); c < nchunks; ++c) {
-                        st = drain(c);
-                        if (st != GZG_OK) return abandon(st);
-                }
-        }
-        for (int k = 0; k < kSlots; ++k) {
-                st = wait_stream(stg->st[k], "batch sync");
-                if (st != GZG_OK) return abandon(st);
+        if (st != GZG_OK) {
+                // A wait that ran out leaves chunks in flight on the staging
+                // streams: their buffers are left to them (never freed nor
+                // pooled again).
+                if (st == GZG_ERR_TIMEOUT) stg.release();
+                return st;
         }
         s->release(std::move(stg));
         uint32_t w = 0;

@@ -1,0 +1,67 @@
+"""The host batch on pageable arrays, which several threads stage in small
+chunks, against the same call on pinned arrays (one thread, copied directly):
+the same bytes at counts around the chunk sizes, for every result format, with
+callers running at once, and a time-out that leaves the scene usable."""
+import threading
+
+import numpy as np
+import pytest
+
+from gonzales_b200 import GpuAccelerator, scenes
+from gonzales_b200 import _ffi as F
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rays():
+    hs = scenes.raycast_scene(subdiv=4).build()
+    n = (1 << 20) + 12345
+    o, d, t = scenes.raycast_rays(hs, 1024, 512, n - 1024 * 512, seed=3)
+    acc = GpuAccelerator(hs)
+    yield acc, scenes.pack_reference_rays(o, d), t
+    acc.close()
+
+
+def _pinned(a):
+    import torch
+
+    return torch.from_numpy(a).pin_memory().numpy()
+
+
+def _direct(acc, r6, t):
+    import torch
+
+    out = torch.zeros(len(t) * F.INTERSECTION_DTYPE.itemsize, dtype=torch.uint8).pin_memory().numpy()
+    return acc.intersect_batch(_pinned(r6), _pinned(t), out=out.view(F.INTERSECTION_DTYPE)).copy()
+
+
+@pytest.mark.parametrize("n", [1, 16383, 16384, 16385, 16384 * 8, 16384 * 16 + 1, (1 << 17) * 8 + 3, (1 << 20) + 12345])
+def test_staged_equals_direct(rays, n):
+    acc, r6, t = rays
+    ref = _direct(acc, r6[:n], t[:n])
+    got = acc.intersect_batch(r6[:n], t[:n])
+    assert got.tobytes() == ref.tobytes()
+    hits = acc.intersect_batch_hits(r6[:n], t[:n])
+    assert hits[:, 0].tobytes() == ref["t_hit"].tobytes()
+    occ = acc.occluded_batch(r6[:n], t[:n])
+    assert np.array_equal(occ, (ref["hit"] != 0).astype(np.uint8))
+    assert acc.error_word() == 0
+
+
+def test_callers_at_once(rays):
+    acc, r6, t = rays
+    n = 300_000
+    ref = acc.intersect_batch(r6[:n], t[:n])
+    got = [None] * 6
+
+    def call(k):
+        got[k] = acc.intersect_batch(r6[k * 1000:n], t[k * 1000:n])
+
+    threads = [threading.Thread(target=call, args=(k,)) for k in range(6)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    for k in range(6):
+        assert got[k].tobytes() == ref[k * 1000:].tobytes()
