@@ -750,6 +750,7 @@ gzg_status upload_scene(const gzg_bvh2_node *bvh2_nodes, int64_t bvh2_node_count
         d.bvh2_count = build ? 0 : bvh2_node_count;
         d.prim_count = prim_count;
         d.wide_count = (uint32_t)wide.nodes.size();
+        d.wide_nodes = d.wide_count;
         d.rcp_max = wide_rcp_max(wide.nodes.data(), wide.nodes.size());
 
         gzg_scene_info &info = scene->info;
@@ -986,6 +987,7 @@ GZG_API gzg_status gzg_gpu_build_mesh_scene(const gzg_mesh_arrays *meshes, int64
         d.bvh2_count = 0;
         d.prim_count = nt;
         d.wide_count = (uint32_t)wide.nodes.size();
+        d.wide_nodes = d.wide_count;
         d.rcp_max = wide_rcp_max(wide.nodes.data(), wide.nodes.size());
         gzg_scene_info &info = scene->info;
         info.bvh2_nodes = 0;
@@ -1544,6 +1546,7 @@ GZG_API gzg_status gzg_instanced_scene_create(gzg_scene *const *blas, int64_t bl
         if ((st = scene->upload(&zero, 1, &ew, "error word"))) return st;
         d.err = const_cast<uint32_t *>(ew);
         d.wide_count = (uint32_t)std::min<uint64_t>(steps, 0xFFFFFFFFull);
+        d.wide_nodes = (uint32_t)nodes.size();
         d.rcp_max = wide_rcp_max(nodes.data(), nodes.size());
         scene->info.wide_nodes = (int64_t)nodes.size();
         scene->info.triangles = (int64_t)(v0.size() - tlas.v0.size());

@@ -24,7 +24,8 @@ struct DevScene {
         const gzg_prim_id *prims;
         int64_t bvh2_count;
         int64_t prim_count;
-        uint32_t wide_count;
+        uint32_t wide_count;  // step cap of a ray: nodes it can open (two-level: over all its instances)
+        uint32_t wide_nodes;  // nodes in the array
         // Bound on |1/direction| in the wide kernels' slab tests: 2^64, or less
         // for scenes of extents above about 2^54 (wide_rcp_max).
         float rcp_max = 18446744073709551616.0f;

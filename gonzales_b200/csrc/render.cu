@@ -2277,6 +2277,7 @@ gzg_status build_batch(gzg_renderer *r) {
                 d.err = err;
                 d.prim_count = (int64_t)prims.size();
                 d.wide_count = (uint32_t)std::min<uint64_t>(steps, 0xFFFFFFFFull);
+                d.wide_nodes = (uint32_t)nodes.size();
                 d.rcp_max = wide_rcp_max(nodes.data(), nodes.size());
                 d.material_count = (int32_t)(mats.size() / 2);
                 d.light_count = (int32_t)(lights.size() / 4);

@@ -469,6 +469,259 @@ __global__ void __launch_bounds__(128, 8) k_wide_persistent(DevScene s, const vo
         }
 }
 
+// Triangle queue of a warp (k_wide_queued, k_wide_instanced_queued): up to 32
+// (record, owner lane) pairs, and the tests' results by queue position.
+struct TriQueue {
+        float4 result[32];  // t, u, v, prim bits; written where the test passed
+        uint2 pair[32];
+};
+
+// Adds the triangles `tris` (bits of tri_bits) of every lane to the queue of
+// `queued` pairs, in lane order, as far as there is room; `have` = the lanes
+// that have some.  The positions a lane's triangles get are added to `mine`.
+// Returns the new length.
+__device__ __forceinline__ uint32_t queue_append(TriQueue &queue, uint32_t queued, unsigned have, uint32_t &tris,
+                                                 uint32_t tri_base, uint32_t tri_bits, uint32_t &mine) {
+        const unsigned FULL = 0xFFFFFFFFu;
+        const unsigned lane = threadIdx.x & 31u;
+        const unsigned lt_mask = (1u << lane) - 1u;
+        uint32_t added;
+        if (__any_sync(FULL, (tris & (tris - 1u)) != 0u)) {
+                // up to 7 a lane at once; the rest is left to the next call
+                const uint32_t count = min(__popc(tris), 7);
+                const unsigned c0 = __ballot_sync(FULL, count & 1u), c1 = __ballot_sync(FULL, count & 2u),
+                               c2 = __ballot_sync(FULL, count & 4u);
+                uint32_t at = queued + __popc(c0 & lt_mask) + 2u * __popc(c1 & lt_mask) + 4u * __popc(c2 & lt_mask);
+                added = __popc(c0) + 2u * __popc(c1) + 4u * __popc(c2);
+                for (const uint32_t last = min(at + count, 32u); at < last; ++at) {
+                        const uint32_t b = __ffs(tris) - 1;
+                        tris &= tris - 1;
+                        queue.pair[at] = make_uint2(tri_record(tri_base, tri_bits, b), lane);
+                        mine |= 1u << at;
+                }
+        } else {
+                const uint32_t at = queued + __popc(have & lt_mask);
+                added = __popc(have);
+                if (tris != 0u && at < 32u) {
+                        queue.pair[at] = make_uint2(tri_record(tri_base, tri_bits, (uint32_t)(__ffs(tris) - 1)), lane);
+                        mine |= 1u << at;
+                        tris = 0u;
+                }
+        }
+        return min(queued + added, 32u);
+}
+
+// Tests the queue's pairs, one per lane, each against its owner's ray and
+// nearest hit so far; the results of the tests that passed (the bits returned)
+// are in queue.result.
+template <int LEAF>
+__device__ __forceinline__ unsigned queue_test(const DevScene &s, TriQueue &queue, uint32_t queued, const WideRay &r,
+                                               float thit) {
+        const unsigned FULL = 0xFFFFFFFFu;
+        const unsigned lane = threadIdx.x & 31u;
+        __syncwarp();
+        const bool test = lane < queued;
+        const uint2 pair = queue.pair[test ? lane : 0u];
+        const int owner = (int)pair.y;
+        const float ox = __shfl_sync(FULL, r.ox, owner), oy = __shfl_sync(FULL, r.oy, owner),
+                    oz = __shfl_sync(FULL, r.oz, owner), dx = __shfl_sync(FULL, r.dx, owner),
+                    dy = __shfl_sync(FULL, r.dy, owner), dz = __shfl_sync(FULL, r.dz, owner);
+        const float limit = __shfl_sync(FULL, thit, owner);
+        bool ok = false;
+        if (test) {
+                count_lanes(s, 1);
+                const float4 a = __ldg(s.tv0 + pair.x);
+                const float4 b = __ldg(s.tv1 + pair.x);
+                const float4 c = __ldg(s.tv2 + pair.x);
+                float t, u, v;
+                ok = leaf_test<LEAF>(ox, oy, oz, dx, dy, dz, a, b, c, limit, t, u, v);
+                if (ok) queue.result[lane] = make_float4(t, u, v, a.w);
+        }
+        const unsigned passed = __ballot_sync(FULL, ok);
+        __syncwarp();
+        return passed;
+}
+
+// Pairs that make a warp test its queue, and rays that only wait for it.  More
+// pairs fill the tests' lanes better but prune later: of 8 to 32 pairs and 2 to
+// 8 rays these were the fastest over camera, incoherent and any-hit rays (8M
+// incoherent rays 1,769 us at 20 pairs and 1,833 at 8 or 32, 8M camera rays 960
+// at 32).
+constexpr int kQueueTests = 12, kQueueWaiting = 3;
+
+// k_wide_persistent with its triangle tests gathered over the warp.  An
+// incoherent warp opens nodes on 29 lanes but finds about six triangles a step,
+// two or three on one lane: testing them lane by lane ran the 90 instructions
+// of a test two or three times a step on two or three lanes.  Here the pairs
+// queue up in shared memory and are tested one per lane, with the owner's ray
+// by shuffle; a ray goes on opening nodes meanwhile, against the nearest hit it
+// knows.  The hits are the same: a triangle is accepted at t <= the nearest t of
+// those before it, and pairs are taken in the order of the nodes.
+// 8M incoherent rays on 1,310,720 triangles 2,116 -> 1,804 us, 4M any-hit rays
+// 892 -> 830, 8M camera rays 918 -> 870, 64 x 64 camera rays on 20,480
+// triangles 41.1 -> 34.8.  launch_trace says where k_wide_persistent stays.
+template <int RAYFMT, int OUTFMT, bool ANY, int STACK, int LEAF>
+__global__ void __launch_bounds__(128, 8) k_wide_queued(DevScene s, const void *__restrict__ rays,
+                                                        const float *__restrict__ tmaxs, int64_t n,
+                                                        void *__restrict__ out) {
+        extern __shared__ __align__(16) uint2 smem_stack[];
+        const unsigned FULL = 0xFFFFFFFFu;
+        const uint32_t nr = (uint32_t)ray_count(s, n);
+        const unsigned lane = threadIdx.x & 31u;
+        const unsigned lt_mask = (1u << lane) - 1u;
+        ChunkCursor cc;
+        chunk_first(cc, nr);
+
+        uint2 *stack = smem_stack + threadIdx.x;
+        const int stride = blockDim.x;
+        TriQueue &queue = reinterpret_cast<TriQueue *>(smem_stack + STACK * blockDim.x)[threadIdx.x >> 5];
+        uint32_t queued = 0;  // pairs in the queue (warp-uniform)
+        uint32_t mine = 0;    // queue positions of this lane's ray
+        int ray_i = -1;
+        WideRay r;
+        float thit = 0.0f, bu = 0.0f, bv = 0.0f;
+        int prim = -1, sp = 0;
+        uint2 group = make_uint2(0u, 0u);
+        uint32_t steps = 0;
+
+        for (;;) {
+                // ---- refill idle lanes from this warp's chunk sequence (warp-uniform cursor)
+                unsigned need = __ballot_sync(FULL, ray_i < 0);
+                if (__popc(need) < kRefillMin && need != FULL) need = 0u;
+                while (need != 0u && cc.cursor < nr) {
+                        if (cc.cursor >= cc.end && !chunk_next(cc, s.sched, nr)) break;
+                        const int avail = (int)(cc.end - cc.cursor);
+                        const int rank = __popc(need & lt_mask);
+                        if (ray_i < 0 && rank < avail) {
+                                ray_i = (int)(cc.cursor + (uint32_t)rank);
+                                const RayIn in = load_ray<RAYFMT>(rays, tmaxs, ray_i);
+                                r.ox = in.ox;
+                                r.oy = in.oy;
+                                r.oz = in.oz;
+                                r.dx = in.dx;
+                                r.dy = in.dy;
+                                r.dz = in.dz;
+                                r.rdx = wide_rcp(in.dx, s.rcp_max);
+                                r.rdy = wide_rcp(in.dy, s.rcp_max);
+                                r.rdz = wide_rcp(in.dz, s.rcp_max);
+                                r.oct = (__float_as_uint(r.rdx) >> 31) | ((__float_as_uint(r.rdy) >> 31) << 1) |
+                                        ((__float_as_uint(r.rdz) >> 31) << 2);
+                                thit = in.tmax;
+                                bu = bv = 0.0f;
+                                prim = -1;
+                                sp = 0;
+                                steps = 0;
+                                group = make_uint2(s.per_ray_root ? in.root : 0u, (1u << 24) | (1u << r.oct));
+                        }
+                        const int npop = __popc(need);
+                        cc.cursor += (uint32_t)(npop < avail ? npop : avail);
+                        need = __ballot_sync(FULL, ray_i < 0);
+                }
+                if (__all_sync(FULL, ray_i < 0)) break;
+
+                // ---- open one node of every ray that has one left; a ray without
+                // hits left in its group takes the next from its stack at once
+                uint32_t tris = 0, tri_base = 0, tri_bits = 0;
+                uint32_t hits = group.y >> 24;
+                if (hits) {
+                        const uint32_t key = __ffs(hits) - 1;
+                        hits &= hits - 1;
+                        const uint32_t im = group.y & 0xFFu;
+                        const uint32_t slot = key ^ r.oct;
+                        const uint32_t node = group.x + __popc(im & ((1u << slot) - 1u));
+                        bool fault = false;
+                        if (hits) {
+                                if (sp >= STACK) {
+                                        atomicOr(s.err, kErrStackOverflow);
+                                        fault = true;
+                                } else {
+                                        stack[sp * stride] = make_uint2(group.x, (hits << 24) | im);
+                                        ++sp;
+                                }
+                        }
+                        if (++steps > s.wide_count) {
+                                atomicOr(s.err, kErrStepCap);
+                                fault = true;
+                        }
+                        group.y = 0u;
+                        if (fault) {
+                                sp = 0;
+                        } else {
+                                const NodeHits h = open_node(s.wide + 5 * (size_t)node, r, thit);
+                                count_lanes(s, 0);
+                                group = make_uint2(h.child_base, (h.nodes << 24) | h.imask);
+                                tris = h.tris;
+                                tri_base = h.tri_base;
+                                tri_bits = h.tri_bits;
+                        }
+                        if ((group.y >> 24) == 0 && sp > 0) {
+                                --sp;
+                                group = stack[sp * stride];
+                        }
+                }
+                __syncwarp();
+
+                // ---- queue the triangles of the leaves hit; test the queue when it
+                // is full enough, or rays only wait for it
+                unsigned have = __ballot_sync(FULL, tris != 0u);
+                while ((have | queued) != 0u) {
+                        if (have != 0u) {
+                                queued = queue_append(queue, queued, have, tris, tri_base, tri_bits, mine);
+                                have = __ballot_sync(FULL, tris != 0u);  // what found no room
+                        }
+                        if (have == 0u && queued < kQueueTests) {
+                                const unsigned busy = __ballot_sync(FULL, (group.y >> 24) != 0u);
+                                const unsigned waiting = __ballot_sync(FULL, (group.y >> 24) == 0u && mine != 0u);
+                                if (busy != 0u && __popc(waiting) < kQueueWaiting) break;
+                        }
+                        uint32_t passed = queue_test<LEAF>(s, queue, queued, r, thit) & mine;
+                        // in queue order, a later triangle at the same t wins
+                        while (passed) {
+                                const uint32_t b = __ffs(passed) - 1;
+                                passed &= passed - 1;
+                                float4 h = queue.result[b];
+                                if (LEAF == GZG_LEAF_WATERTIGHT) {
+                                        // its limit is rounded with the triangle's
+                                        // determinant: tested again against the
+                                        // hits before it
+                                        const uint32_t ti = queue.pair[b].x;
+                                        if (!leaf_test<LEAF>(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, __ldg(s.tv0 + ti),
+                                                             __ldg(s.tv1 + ti), __ldg(s.tv2 + ti), thit, h.x, h.y, h.z))
+                                                continue;
+                                } else if (!(h.x <= thit)) {
+                                        continue;
+                                }
+                                thit = h.x;
+                                bu = h.y;
+                                bv = h.z;
+                                prim = __float_as_int(h.w);
+                                if (ANY) {
+                                        tris = 0u;
+                                        break;  // the first one, whatever was tested with it
+                                }
+                        }
+                        __syncwarp();
+                        mine = 0u;
+                        queued = 0u;
+                        if (ANY) have = __ballot_sync(FULL, tris != 0u);
+                }
+                if (ray_i >= 0 && mine == 0u && (ANY ? prim >= 0 || (group.y >> 24) == 0u : (group.y >> 24) == 0u)) {
+                        if (prim < 0) {
+                                // a miss reports the ray's tMax, read again
+                                // rather than kept in a register
+                                thit = load_ray<RAYFMT>(rays, tmaxs, ray_i).tmax;
+                                bu = 0.0f;
+                                bv = 0.0f;
+                        }
+                        store_hit<OUTFMT>(s, out, ray_i, prim, thit, bu, bv);
+                        ray_i = -1;
+                        group.y = 0u;
+                        sp = 0;
+                        count_lanes(s, 2);
+                }
+        }
+}
+
 __device__ __forceinline__ void set_ray_dirs(WideRay &r, float limit) {
         r.rdx = wide_rcp(r.dx, limit);
         r.rdy = wide_rcp(r.dy, limit);
@@ -698,6 +951,236 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced(DevScene s, const voi
         }
 }
 
+constexpr int kQueueTestsInst = 12, kQueueWaitingInst = 4;
+
+// k_wide_instanced with the triangle queue of k_wide_queued.  The top level's
+// leaves hold instances only and the bottom levels' triangles only, so an
+// instance is entered where its record is met and triangles are queued; a ray
+// whose triangles are still queued waits before it leaves its instance, because
+// they are tested with its object-space ray.  2M rays through 4096 instances
+// 1,359 -> 1,215 us, two-level frame 26.2 -> 24.4 ms.
+template <int OUTFMT, bool ANY, int STACK>
+__global__ void __launch_bounds__(128, 8) k_wide_instanced_queued(DevScene s, const void *__restrict__ rays,
+                                                                  const float *__restrict__ tmaxs, int64_t n,
+                                                                  void *__restrict__ out) {
+        extern __shared__ __align__(16) uint2 smem_stack[];
+        const unsigned FULL = 0xFFFFFFFFu;
+        const uint32_t nr = (uint32_t)ray_count(s, n);
+        const unsigned lane = threadIdx.x & 31u;
+        const unsigned lt_mask = (1u << lane) - 1u;
+        ChunkCursor cc;
+        chunk_first(cc, nr);
+
+        uint2 *stack = smem_stack + threadIdx.x;
+        const int stride = blockDim.x;
+        TriQueue &queue = reinterpret_cast<TriQueue *>(smem_stack + STACK * blockDim.x)[threadIdx.x >> 5];
+        uint32_t queued = 0;  // pairs in the queue (warp-uniform)
+        uint32_t mine = 0;    // queue positions of this lane's ray
+        int ray_i = -1;
+        WideRay r;
+        float thit = 0.0f, bu = 0.0f, bv = 0.0f;
+        int prim = -1, hit_inst = -1, cur_inst = -1, sp = 0;
+        uint2 group = make_uint2(0u, 0u);
+        uint32_t steps = 0;
+
+        for (;;) {
+                unsigned need = __ballot_sync(FULL, ray_i < 0);
+                if (__popc(need) < kRefillMin && need != FULL) need = 0u;
+                while (need != 0u && cc.cursor < nr) {
+                        if (cc.cursor >= cc.end && !chunk_next(cc, s.sched, nr)) break;
+                        const int avail = (int)(cc.end - cc.cursor);
+                        const int rank = __popc(need & lt_mask);
+                        if (ray_i < 0 && rank < avail) {
+                                ray_i = (int)(cc.cursor + (uint32_t)rank);
+                                const RayIn in = load_ray<kRayDevice>(rays, tmaxs, ray_i);
+                                r.ox = in.ox;
+                                r.oy = in.oy;
+                                r.oz = in.oz;
+                                r.dx = in.dx;
+                                r.dy = in.dy;
+                                r.dz = in.dz;
+                                set_ray_dirs(r, s.rcp_max);
+                                thit = in.tmax;
+                                bu = bv = 0.0f;
+                                prim = hit_inst = cur_inst = -1;
+                                sp = 0;
+                                steps = 0;
+                                group = make_uint2(0u, (1u << 24) | (1u << r.oct));
+                        }
+                        const int npop = __popc(need);
+                        cc.cursor += (uint32_t)(npop < avail ? npop : avail);
+                        need = __ballot_sync(FULL, ray_i < 0);
+                }
+                if (__all_sync(FULL, ray_i < 0)) break;
+
+                // top-level leaf records to enter: bits pend_mask of pend_bits
+                uint32_t pend_base = 0, pend_bits = 0, pend_mask = 0;
+                // bottom-level triangles to queue
+                uint32_t tris = 0, tri_base = 0, tri_bits = 0;
+                bool fault = false, waits = false;
+                // pop until there is work: a world-ray marker restores the world
+                // ray and pops again in the same step, unless the queue still
+                // holds triangles of the instance
+                while ((group.y >> 24) == 0 && sp > 0) {
+                        const uint2 e = stack[(sp - 1) * stride];
+                        if (e.x == 0xFFFFFFFFu) {
+                                if (mine != 0u) {
+                                        waits = true;
+                                        break;
+                                }
+                                --sp;
+                                world_ray(rays, ray_i, r);
+                                set_ray_dirs(r, s.rcp_max);
+                                cur_inst = -1;
+                        } else {
+                                --sp;
+                                if (e.x & 0x80000000u) {
+                                        pend_base = e.x & 0x7FFFFFFFu;
+                                        pend_mask = e.y;
+                                        pend_bits = 0xFFFFFFFFu;
+                                        break;
+                                }
+                                group = e;
+                        }
+                }
+                uint32_t hits = group.y >> 24;
+                if (pend_mask == 0 && hits) {
+                        const uint32_t key = __ffs(hits) - 1;
+                        hits &= hits - 1;
+                        const uint32_t im = group.y & 0xFFu;
+                        const uint32_t slot = key ^ r.oct;
+                        const uint32_t node = group.x + __popc(im & ((1u << slot) - 1u));
+                        if (hits) {
+                                if (sp >= STACK) {
+                                        atomicOr(s.err, kErrStackOverflow);
+                                        fault = true;
+                                } else {
+                                        stack[sp * stride] = make_uint2(group.x, (hits << 24) | im);
+                                        ++sp;
+                                }
+                        }
+                        if (++steps > s.wide_count) {
+                                atomicOr(s.err, kErrStepCap);
+                                fault = true;
+                        }
+                        if (!fault) {
+                                const NodeHits h = open_node(s.wide + 5 * (size_t)node, r, thit);
+                                count_lanes(s, 0);
+                                group = make_uint2(h.child_base, (h.nodes << 24) | h.imask);
+                                if (cur_inst < 0) {
+                                        // the top level's leaves hold instances,
+                                        // the bottom levels' triangles
+                                        pend_mask = h.tris;
+                                        pend_base = h.tri_base;
+                                        pend_bits = h.tri_bits;
+                                } else {
+                                        tris = h.tris;
+                                        tri_base = h.tri_base;
+                                        tri_bits = h.tri_bits;
+                                }
+                        }
+                }
+                if (pend_mask && !fault) {
+                        // instance record: save the resume state and descend
+                        const uint32_t b = __ffs(pend_mask) - 1;
+                        pend_mask &= pend_mask - 1;
+                        const int inst = -__float_as_int(__ldg(&s.tv0[tri_record(pend_base, pend_bits, b)].w)) - 1;
+                        const int need_slots = ((group.y >> 24) ? 1 : 0) + (pend_mask ? 1 : 0) + 1;
+                        if (sp + need_slots > STACK || (uint32_t)inst >= (uint32_t)s.instance_count) {
+                                atomicOr(s.err, (uint32_t)inst >= (uint32_t)s.instance_count ? kErrBadIndex : kErrStackOverflow);
+                                fault = true;
+                        } else {
+                                if (group.y >> 24) {
+                                        stack[sp * stride] = group;
+                                        ++sp;
+                                }
+                                if (pend_mask) {
+                                        // the records left, as plain offsets from pend_base
+                                        uint32_t left = 0;
+                                        while (pend_mask) {
+                                                const uint32_t q = __ffs(pend_mask) - 1;
+                                                pend_mask &= pend_mask - 1;
+                                                left |= 1u << __popc(pend_bits & ((1u << q) - 1u));
+                                        }
+                                        stack[sp * stride] = make_uint2(0x80000000u | pend_base, left);
+                                        ++sp;
+                                }
+                                stack[sp * stride] = make_uint2(0xFFFFFFFFu, 0u);
+                                ++sp;
+                                const float4 m0 = __ldg(s.instances + 4 * inst), m1 = __ldg(s.instances + 4 * inst + 1),
+                                             m2 = __ldg(s.instances + 4 * inst + 2), m3 = __ldg(s.instances + 4 * inst + 3);
+                                WideRay w;
+                                world_ray(rays, ray_i, w);
+                                r.ox = xf_point(m0, w.ox, w.oy, w.oz);
+                                r.oy = xf_point(m1, w.ox, w.oy, w.oz);
+                                r.oz = xf_point(m2, w.ox, w.oy, w.oz);
+                                r.dx = xf_vector(m0, w.dx, w.dy, w.dz);
+                                r.dy = xf_vector(m1, w.dx, w.dy, w.dz);
+                                r.dz = xf_vector(m2, w.dx, w.dy, w.dz);
+                                set_ray_dirs(r, s.rcp_max);
+                                cur_inst = inst;
+                                group = make_uint2((uint32_t)__float_as_int(m3.x), (1u << 24) | (1u << r.oct));
+                        }
+                }
+                if (fault) {
+                        group.y = 0u;
+                        sp = 0;
+                        tris = 0u;
+                }
+                waits = waits || (ray_i >= 0 && (group.y >> 24) == 0u && sp == 0 && (mine | tris) != 0u);
+                __syncwarp();
+                // queue the triangles; test the queue when it is full enough, or
+                // rays wait for it
+                unsigned have = __ballot_sync(FULL, tris != 0u);
+                while ((have | queued) != 0u) {
+                        if (have != 0u) {
+                                queued = queue_append(queue, queued, have, tris, tri_base, tri_bits, mine);
+                                have = __ballot_sync(FULL, tris != 0u);  // what found no room
+                        }
+                        if (have == 0u && queued < kQueueTestsInst) {
+                                const unsigned waiting = __ballot_sync(FULL, waits);
+                                const unsigned busy = __ballot_sync(FULL, ray_i >= 0 && !waits);
+                                if (busy != 0u && __popc(waiting) < kQueueWaitingInst) break;
+                        }
+                        uint32_t passed = queue_test<GZG_LEAF_MOLLER_TRUMBORE>(s, queue, queued, r, thit) & mine;
+                        while (passed) {
+                                const uint32_t b = __ffs(passed) - 1;
+                                passed &= passed - 1;
+                                const float4 h = queue.result[b];
+                                if (h.x <= thit) {
+                                        thit = h.x;
+                                        bu = h.y;
+                                        bv = h.z;
+                                        prim = __float_as_int(h.w);
+                                        hit_inst = cur_inst;
+                                        if (ANY) {
+                                                tris = 0u;
+                                                break;
+                                        }
+                                }
+                        }
+                        __syncwarp();
+                        mine = 0u;
+                        queued = 0u;
+                        if (ANY) have = __ballot_sync(FULL, tris != 0u);
+                }
+                if (ray_i >= 0 && mine == 0u && ((ANY && prim >= 0) || ((group.y >> 24) == 0u && sp == 0))) {
+                        if (prim < 0) {
+                                thit = load_ray<kRayDevice>(rays, tmaxs, ray_i).tmax;
+                                bu = 0.0f;
+                                bv = 0.0f;
+                                hit_inst = -1;
+                        }
+                        store_hit<OUTFMT>(s, out, ray_i, prim, thit, bu, bv);
+                        if (s.inst_out) s.inst_out[ray_i] = hit_inst;
+                        ray_i = -1;
+                        group.y = 0u;
+                        sp = 0;
+                        count_lanes(s, 2);
+                }
+        }
+}
+
 // The reference's slab test (kernel.mojo:171-206), separately rounded.
 __device__ __forceinline__ bool ref_aabb(const float4 &lo, const float4 &hi, const float rd[3], const float ord[3],
                                          const bool nm[3], float tmax, float &tnear_out) {
@@ -832,13 +1315,13 @@ using TraceKernel = void (*)(DevScene, const void *, const float *, int64_t, voi
 // SM, from the occupancy calculator unless blocks_per_sm is given), capped at
 // the blocks the ray count needs; the one-ray-per-thread kernel one thread per
 // ray.
-cudaError_t launch_wide_kernel(TraceKernel k, int stack, bool persistent, const LaunchParams &p, const DevScene &s,
+cudaError_t launch_wide_kernel(TraceKernel k, int stack, bool persistent, bool queued, const LaunchParams &p, const DevScene &s,
                                const void *rays, const float *tmax, int64_t n, void *out, cudaStream_t st) {
         // The persistent kernel is compiled for blocks of at most 128 threads
         // (measured faster for any-hit queries than a 256-thread bound).
         const int block = (p.block_size == 64 || (p.block_size == 256 && !persistent)) ? p.block_size : 128;
         const int blocks_per_sm = p.blocks_per_sm;
-        const size_t smem = (size_t)stack * block * sizeof(uint2);
+        const size_t smem = (size_t)stack * block * sizeof(uint2) + (queued ? (size_t)(block / 32) * sizeof(TriQueue) : 0);
         if (smem > 48 * 1024) {
                 cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 if (e != cudaSuccess) return e;
@@ -879,30 +1362,55 @@ cudaError_t launch_wide_kernel(TraceKernel k, int stack, bool persistent, const 
         return cudaGetLastError();
 }
 
+// Whether a launch of n rays over a wide tree of `nodes` nodes tests triangles
+// lane by lane (k_wide_persistent, k_wide_instanced) instead of through the
+// warp's queue.  Where many rays meet each triangle, neighbouring rays meet it
+// in the same step and the lanes are full as they are: pinhole rays are slower
+// with the queue above about 80 rays a triangle, 400 a node (8.4M rays on 1,280
+// triangles 448 -> 491 us, on 20,480 585 -> 605, on 81,920 681 -> 685; 0.5M on
+// 5,120 83.4 -> 83.9), and faster below (0.5M rays on 20,480 triangles 105.3 ->
+// 101.5, 8.4M on 1,310,720 918 -> 871).  Incoherent rays would be faster with
+// it on small trees too (0.4M on 1,280 triangles 86 -> 77 us), but a launch
+// does not know its rays.
+bool lane_tests(int64_t n, uint32_t nodes) { return n > 400 * (int64_t)nodes; }
+
+template <int RAYFMT, int OUTFMT, bool ANY, int STACK, int LEAF>
+cudaError_t launch_wide_stack(const DevScene &s, const LaunchParams &p, const void *rays, const float *tmax, int64_t n,
+                              void *out, cudaStream_t st) {
+        if (p.traversal != GZG_TRAVERSAL_WIDE)
+                return launch_wide_kernel(k_wide<RAYFMT, OUTFMT, ANY, STACK, LEAF>, STACK, false, false, p, s, rays, tmax, n, out, st);
+        // (a tree too deep for 16 entries has too many nodes for the other kernel to matter)
+        if constexpr (STACK <= 16)
+                if (lane_tests(n, s.wide_nodes))
+                        return launch_wide_kernel(k_wide_persistent<RAYFMT, OUTFMT, ANY, STACK, LEAF>, STACK, true, false, p, s,
+                                                  rays, tmax, n, out, st);
+        return launch_wide_kernel(k_wide_queued<RAYFMT, OUTFMT, ANY, STACK, LEAF>, STACK, true, true, p, s, rays, tmax, n, out, st);
+}
+
 template <int RAYFMT, int OUTFMT, bool ANY, int LEAF>
 cudaError_t launch_wide_depth(const DevScene &s, const LaunchParams &p, const void *rays, const float *tmax, int64_t n,
                               void *out, cudaStream_t st) {
-        const bool persistent = p.traversal == GZG_TRAVERSAL_WIDE;
         // A ray pushes at most one group (the rest of a node's interior hits)
         // per level whose nodes have interior children, so the stack holds at
         // most depth - 1 groups; a requested depth below that is raised so no
         // ray can overflow it (an overflow would set kErrStackOverflow).
         const int need = p.wide_depth > 2 ? p.wide_depth - 1 : 1;
         const int want = p.stack_depth > need ? p.stack_depth : need;
-        if (want <= 8) {
-                TraceKernel k = persistent ? k_wide_persistent<RAYFMT, OUTFMT, ANY, 8, LEAF> : k_wide<RAYFMT, OUTFMT, ANY, 8, LEAF>;
-                return launch_wide_kernel(k, 8, persistent, p, s, rays, tmax, n, out, st);
-        }
-        if (want <= 16) {
-                TraceKernel k = persistent ? k_wide_persistent<RAYFMT, OUTFMT, ANY, 16, LEAF> : k_wide<RAYFMT, OUTFMT, ANY, 16, LEAF>;
-                return launch_wide_kernel(k, 16, persistent, p, s, rays, tmax, n, out, st);
-        }
-        if (want <= 32) {
-                TraceKernel k = persistent ? k_wide_persistent<RAYFMT, OUTFMT, ANY, 32, LEAF> : k_wide<RAYFMT, OUTFMT, ANY, 32, LEAF>;
-                return launch_wide_kernel(k, 32, persistent, p, s, rays, tmax, n, out, st);
-        }
-        TraceKernel k = persistent ? k_wide_persistent<RAYFMT, OUTFMT, ANY, 64, LEAF> : k_wide<RAYFMT, OUTFMT, ANY, 64, LEAF>;
-        return launch_wide_kernel(k, 64, persistent, p, s, rays, tmax, n, out, st);
+        if (want <= 8) return launch_wide_stack<RAYFMT, OUTFMT, ANY, 8, LEAF>(s, p, rays, tmax, n, out, st);
+        if (want <= 16) return launch_wide_stack<RAYFMT, OUTFMT, ANY, 16, LEAF>(s, p, rays, tmax, n, out, st);
+        if (want <= 32) return launch_wide_stack<RAYFMT, OUTFMT, ANY, 32, LEAF>(s, p, rays, tmax, n, out, st);
+        return launch_wide_stack<RAYFMT, OUTFMT, ANY, 64, LEAF>(s, p, rays, tmax, n, out, st);
+}
+
+template <int STACK>
+cudaError_t launch_instanced_stack(const DevScene &s, const LaunchParams &p, int out_fmt, const void *rays, int64_t n,
+                                   void *out, cudaStream_t st) {
+        const bool lanes = lane_tests(n, s.wide_nodes);
+        const TraceKernel k =
+            out_fmt == kOutHit    ? (lanes ? k_wide_instanced<kOutHit, false, STACK> : k_wide_instanced_queued<kOutHit, false, STACK>)
+            : out_fmt == kOutShadow ? (lanes ? k_wide_instanced<kOutShadow, true, STACK> : k_wide_instanced_queued<kOutShadow, true, STACK>)
+                                    : (lanes ? k_wide_instanced<kOutAnyPrim, true, STACK> : k_wide_instanced_queued<kOutAnyPrim, true, STACK>);
+        return launch_wide_kernel(k, STACK, true, !lanes, p, s, rays, nullptr, n, out, st);
 }
 
 template <int RAYFMT, int OUTFMT, bool ANY>
@@ -958,37 +1466,14 @@ cudaError_t launch_trace(const DevScene &scene, const LaunchParams &p, int ray_f
                 const int want = p.stack_depth > need ? p.stack_depth : need;
                 LaunchParams q = p;
                 q.traversal = GZG_TRAVERSAL_WIDE;
-                TraceKernel k;
-                int stack;
-                if (want <= 16) {
-                        stack = 16;
-                        k = out_fmt == kOutHit ? k_wide_instanced<kOutHit, false, 16>
-                            : out_fmt == kOutShadow ? k_wide_instanced<kOutShadow, true, 16>
-                                                    : k_wide_instanced<kOutAnyPrim, true, 16>;
-                } else if (want <= 32) {
-                        stack = 32;
-                        k = out_fmt == kOutHit ? k_wide_instanced<kOutHit, false, 32>
-                            : out_fmt == kOutShadow ? k_wide_instanced<kOutShadow, true, 32>
-                                                    : k_wide_instanced<kOutAnyPrim, true, 32>;
-                } else {
-                        stack = 64;
-                        k = out_fmt == kOutHit ? k_wide_instanced<kOutHit, false, 64>
-                            : out_fmt == kOutShadow ? k_wide_instanced<kOutShadow, true, 64>
-                                                    : k_wide_instanced<kOutAnyPrim, true, 64>;
-                }
-                return launch_wide_kernel(k, stack, true, q, s, rays, tmax, n, out, st);
+                if (want <= 16) return launch_instanced_stack<16>(s, q, out_fmt, rays, n, out, st);
+                if (want <= 32) return launch_instanced_stack<32>(s, q, out_fmt, rays, n, out, st);
+                return launch_instanced_stack<64>(s, q, out_fmt, rays, n, out, st);
         }
         if (out_fmt == kOutShadow) {
                 // a renderer's shadow queue: one traversal, one leaf test
-                if (ray_fmt != kRayDevice) return cudaErrorNotSupported;
-                const int need = p.wide_depth > 2 ? p.wide_depth - 1 : 1;
-                const int want = p.stack_depth > need ? p.stack_depth : need;
-                const TraceKernel k = want <= 8    ? k_wide_persistent<kRayDevice, kOutShadow, true, 8, GZG_LEAF_MOLLER_TRUMBORE>
-                                      : want <= 16 ? k_wide_persistent<kRayDevice, kOutShadow, true, 16, GZG_LEAF_MOLLER_TRUMBORE>
-                                      : want <= 32 ? k_wide_persistent<kRayDevice, kOutShadow, true, 32, GZG_LEAF_MOLLER_TRUMBORE>
-                                                   : k_wide_persistent<kRayDevice, kOutShadow, true, 64, GZG_LEAF_MOLLER_TRUMBORE>;
-                const int stack = want <= 8 ? 8 : want <= 16 ? 16 : want <= 32 ? 32 : 64;
-                return launch_wide_kernel(k, stack, true, p, s, rays, tmax, n, out, st);
+                if (ray_fmt != kRayDevice || p.traversal != GZG_TRAVERSAL_WIDE) return cudaErrorNotSupported;
+                return launch_wide_depth<kRayDevice, kOutShadow, true, GZG_LEAF_MOLLER_TRUMBORE>(s, p, rays, tmax, n, out, st);
         }
         if (ray_fmt == kRayDevice) {
                 switch (out_fmt) {
