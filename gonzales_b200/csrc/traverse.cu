@@ -688,7 +688,7 @@ __global__ void __launch_bounds__(128, 8) k_wide_queued(DevScene s, const void *
                                         if (!leaf_test<LEAF>(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, __ldg(s.tv0 + ti),
                                                              __ldg(s.tv1 + ti), __ldg(s.tv2 + ti), thit, h.x, h.y, h.z))
                                                 continue;
-                                } else if (!(h.x <= thit)) {
+                                } else if (h.x > thit) {  // as mt_test: a NaN limit or distance accepts
                                         continue;
                                 }
                                 thit = h.x;
@@ -1147,16 +1147,15 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced_queued(DevScene s, co
                                 const uint32_t b = __ffs(passed) - 1;
                                 passed &= passed - 1;
                                 const float4 h = queue.result[b];
-                                if (h.x <= thit) {
-                                        thit = h.x;
-                                        bu = h.y;
-                                        bv = h.z;
-                                        prim = __float_as_int(h.w);
-                                        hit_inst = cur_inst;
-                                        if (ANY) {
-                                                tris = 0u;
-                                                break;
-                                        }
+                                if (h.x > thit) continue;  // as mt_test: a NaN limit or distance accepts
+                                thit = h.x;
+                                bu = h.y;
+                                bv = h.z;
+                                prim = __float_as_int(h.w);
+                                hit_inst = cur_inst;
+                                if (ANY) {
+                                        tris = 0u;
+                                        break;
                                 }
                         }
                         __syncwarp();

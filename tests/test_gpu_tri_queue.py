@@ -102,3 +102,66 @@ def test_two_level_queue_equals_lane_tests(n_instances):
         assert acc.error_word() == 0
     for b in blas:
         b.close()
+
+
+def _both_ways(acc, rays, n, opt, step):
+    """Closest hits and first prims of one launch (lane tests) and of slices (queue)."""
+    import torch
+
+    hits = [torch.empty((n, 4), device="cuda") for _ in range(2)]
+    prim = [torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2)]
+    acc.trace_closest(rays, hits[0], opt)
+    acc.trace_any(rays, prim[0], opt)
+    for s in _slices(n, step):
+        acc.trace_closest(rays[s], hits[1][s], opt)
+        acc.trace_any(rays[s], prim[1][s], opt)
+    torch.cuda.synchronize()
+    return [h.cpu().numpy() for h in hits], [p.cpu().numpy() for p in prim]
+
+
+@pytest.mark.parametrize("kind", ["9", "grid"])
+@pytest.mark.parametrize("leaf", [F.LEAF_MOLLER_TRUMBORE, F.LEAF_WATERTIGHT])
+def test_a_nan_limit_gives_one_answer(kind, leaf):
+    """A ray whose tMax is NaN is limited by nothing in the leaf tests; the
+    queue, the lane tests and the one-ray-per-thread kernel say the same."""
+    import torch
+
+    rng = np.random.default_rng(7)
+    with GpuAccelerator(_edge_scene(kind, rng)) as acc:
+        nodes = acc.info()["wide_nodes"]
+        n = 400 * nodes + 777
+        host = _rays(rng, n)
+        host[::3, 3] = np.nan
+        rays = torch.from_numpy(host).cuda()
+        hits, prim = _both_ways(acc, rays, n, options(leaf_test=leaf), 1 + 130 * nodes)
+        assert hits[0].tobytes() == hits[1].tobytes()
+        assert np.array_equal(prim[0], prim[1])
+        one = torch.empty((n, 4), device="cuda")
+        acc.trace_closest(rays, one, options(leaf_test=leaf, traversal=F.TRAVERSAL_WIDE_ONE_RAY_PER_THREAD))
+        torch.cuda.synchronize()
+        assert one.cpu().numpy().tobytes() == hits[0].tobytes()
+        nan = np.isnan(host[:, 3])
+        assert (hits[0][nan, 3].view(np.int32) >= 0).any()
+
+
+def test_two_level_nan_limit_gives_one_answer():
+    import torch
+
+    rng = np.random.default_rng(8)
+    hosts, _ = scenes.instanced_scene(n_meshes=2, n_u=5, n_v=4, n_instances=1)
+    blas = [GpuAccelerator(h) for h in hosts]
+    with InstancedAccelerator(blas, scenes.random_instances(7, 2, 5, extent=1.5)) as acc:
+        n = 400 * acc.info()["wide_nodes"] + 555
+        host = _rays(rng, n, 1.5)
+        host[::3, 3] = np.nan
+        rays = torch.from_numpy(host).cuda()
+        hits = [torch.empty((n, 4), device="cuda") for _ in range(2)]
+        inst = [torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2)]
+        acc.trace_closest(rays, hits[0], inst[0])
+        for s in _slices(n, 1 + n // 5):
+            acc.trace_closest(rays[s], hits[1][s], inst[1][s])
+        torch.cuda.synchronize()
+        assert hits[0].cpu().numpy().tobytes() == hits[1].cpu().numpy().tobytes()
+        assert torch.equal(inst[0], inst[1]) and bool((inst[0][::3] >= 0).any())
+    for b in blas:
+        b.close()
