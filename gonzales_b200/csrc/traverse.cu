@@ -119,8 +119,11 @@ __device__ __forceinline__ F2 qbytes(uint32_t wa, uint32_t wb, uint32_t sel) {
 struct WideRay {
         float ox, oy, oz, dx, dy, dz;
         float rdx, rdy, rdz;
-        uint32_t oct;  // sign bits of the inverse direction
+        uint32_t oct;  // sign bits of the inverse direction; queued kernels: and kAlone
 };
+
+// A ray whose triangles are tested as soon as their node is opened (k_wide_queued).
+constexpr uint32_t kAlone = 8u;
 
 // What a ray hits in a wide node.
 struct NodeHits {
@@ -476,19 +479,28 @@ struct TriQueue {
         uint2 pair[32];
 };
 
+// The two-level kernel has no registers left for what only the end of a ray reads
+// (2M rays through 4096 instances 1,298 us with it in registers, 1,219 here; the
+// one-level kernel is 2 % faster with registers).
+struct InstQueue : TriQueue {
+        float2 uv[32];  // u, v of each lane's nearest hit
+        int inst[32];   // its instance
+};
+
 // Adds the triangles `tris` (bits of tri_bits) of every lane to the queue of
 // `queued` pairs, in lane order, as far as there is room; `have` = the lanes
-// that have some.  The positions a lane's triangles get are added to `mine`.
-// Returns the new length.
+// that have some, and a lane adds `most` at a time.  The positions a lane's
+// triangles get are added to `mine`.  Returns the new length.
 __device__ __forceinline__ uint32_t queue_append(TriQueue &queue, uint32_t queued, unsigned have, uint32_t &tris,
-                                                 uint32_t tri_base, uint32_t tri_bits, uint32_t &mine) {
+                                                 uint32_t tri_base, uint32_t tri_bits, uint32_t &mine, int most) {
         const unsigned FULL = 0xFFFFFFFFu;
         const unsigned lane = threadIdx.x & 31u;
         const unsigned lt_mask = (1u << lane) - 1u;
         uint32_t added;
         if (__any_sync(FULL, (tris & (tris - 1u)) != 0u)) {
-                // up to 7 a lane at once; the rest is left to the next call
-                const uint32_t count = min(__popc(tris), 7);
+                // up to 7 a lane at once, counted by three ballots; the rest is
+                // left to the next call
+                const uint32_t count = min(__popc(tris), most);
                 const unsigned c0 = __ballot_sync(FULL, count & 1u), c1 = __ballot_sync(FULL, count & 2u),
                                c2 = __ballot_sync(FULL, count & 4u);
                 uint32_t at = queued + __popc(c0 & lt_mask) + 2u * __popc(c1 & lt_mask) + 4u * __popc(c2 & lt_mask);
@@ -542,6 +554,27 @@ __device__ __forceinline__ unsigned queue_test(const DevScene &s, TriQueue &queu
         return passed;
 }
 
+// Whether a ray that prunes at once would test triangle ti too, which the queue
+// accepted at t, at most the nearest hit before it: every box above the triangle
+// is entered before t.  Those boxes hold the triangle's own bounds with a margin
+// of 2^-18 of the coordinates; half of it is used here, half is left to rounding.
+// A box's distance and the one here come from the same reciprocals and differ by
+// at most 3.5 x 2^-23 of themselves, 4.2 x 2^-23 is forgiven here, and open_node
+// forgives 9.
+__device__ __forceinline__ float tri_entry_axis(float o, float rd, float a, float b, float c) {
+        const float lo = fminf(a, fminf(b, c)), hi = fmaxf(a, fmaxf(b, c));
+        const float margin = fmaxf(fabsf(lo), fabsf(hi)) * 1.9073486e-6f;  // 2^-19
+        return ((rd < 0.0f ? hi + margin : lo - margin) - o) * rd;
+}
+
+__device__ __forceinline__ bool box_before(const DevScene &s, const WideRay &r, uint32_t ti, float t) {
+        const float4 a = __ldg(s.tv0 + ti), b = __ldg(s.tv1 + ti), c = __ldg(s.tv2 + ti);
+        const float entry = fmaxf(tri_entry_axis(r.ox, r.rdx, a.x, b.x, c.x),
+                                  fmaxf(tri_entry_axis(r.oy, r.rdy, a.y, b.y, c.y),
+                                        tri_entry_axis(r.oz, r.rdz, a.z, b.z, c.z)));
+        return entry <= t * 1.0000005f;
+}
+
 // Pairs that make a warp test its queue, and rays that only wait for it.  More
 // pairs fill the tests' lanes better but prune later: of 8 to 32 pairs and 2 to
 // 8 rays these were the fastest over camera, incoherent and any-hit rays (8M
@@ -555,11 +588,19 @@ constexpr int kQueueTests = 12, kQueueWaiting = 3;
 // of a test two or three times a step on two or three lanes.  Here the pairs
 // queue up in shared memory and are tested one per lane, with the owner's ray
 // by shuffle; a ray goes on opening nodes meanwhile, against the nearest hit it
-// knows.  The hits are the same: a triangle is accepted at t <= the nearest t of
-// those before it, and pairs are taken in the order of the nodes.
-// 8M incoherent rays on 1,310,720 triangles 2,116 -> 1,804 us, 4M any-hit rays
-// 892 -> 830, 8M camera rays 918 -> 870, 64 x 64 camera rays on 20,480
-// triangles 41.1 -> 34.8.  launch_trace says where k_wide_persistent stays.
+// knows.  The hits are those of k_wide_persistent: a triangle is accepted at
+// t <= the nearest t of those before it, and pairs are taken in the order of the
+// nodes.  Nodes opened before a hit in the queue is known add triangles that
+// k_wide_persistent would not test; one of them can only be accepted if its
+// computed t falls before its own boxes (slivers, rays along a surface), if a t
+// is NaN, or if the watertight test's rounded limit let a t above the limit in.
+// Such a ray starts over with its triangles tested one by one as their node is
+// opened (kAlone), so its hit depends on the ray alone and not on its warp
+// (2 to 3 % of a launch: 8M incoherent rays 1,802 -> 1,841 us, 8M camera rays
+// 869 -> 889).
+// Against k_wide_persistent: 8M incoherent rays on 1,310,720 triangles 2,116 ->
+// 1,841 us, 4M any-hit rays 892 -> 830, 8M camera rays 918 -> 889, 64 x 64 camera
+// rays on 20,480 triangles 41.1 -> 35.9.  launch_trace says where k_wide_persistent stays.
 template <int RAYFMT, int OUTFMT, bool ANY, int STACK, int LEAF>
 __global__ void __launch_bounds__(128, 8) k_wide_queued(DevScene s, const void *__restrict__ rays,
                                                         const float *__restrict__ tmaxs, int64_t n,
@@ -627,7 +668,7 @@ __global__ void __launch_bounds__(128, 8) k_wide_queued(DevScene s, const void *
                         const uint32_t key = __ffs(hits) - 1;
                         hits &= hits - 1;
                         const uint32_t im = group.y & 0xFFu;
-                        const uint32_t slot = key ^ r.oct;
+                        const uint32_t slot = (key ^ r.oct) & 7u;
                         const uint32_t node = group.x + __popc(im & ((1u << slot) - 1u));
                         bool fault = false;
                         if (hits) {
@@ -666,30 +707,38 @@ __global__ void __launch_bounds__(128, 8) k_wide_queued(DevScene s, const void *
                 unsigned have = __ballot_sync(FULL, tris != 0u);
                 while ((have | queued) != 0u) {
                         if (have != 0u) {
-                                queued = queue_append(queue, queued, have, tris, tri_base, tri_bits, mine);
+                                queued = queue_append(queue, queued, have, tris, tri_base, tri_bits, mine,
+                                                      !ANY && (r.oct & kAlone) ? 1 : 7);
                                 have = __ballot_sync(FULL, tris != 0u);  // what found no room
                         }
-                        if (have == 0u && queued < kQueueTests) {
+                        if (have == 0u && queued < kQueueTests &&
+                            (ANY || !__any_sync(FULL, (r.oct & kAlone) && mine != 0u))) {
                                 const unsigned busy = __ballot_sync(FULL, (group.y >> 24) != 0u);
                                 const unsigned waiting = __ballot_sync(FULL, (group.y >> 24) == 0u && mine != 0u);
                                 if (busy != 0u && __popc(waiting) < kQueueWaiting) break;
                         }
+                        bool again = false;
                         uint32_t passed = queue_test<LEAF>(s, queue, queued, r, thit) & mine;
                         // in queue order, a later triangle at the same t wins
                         while (passed) {
                                 const uint32_t b = __ffs(passed) - 1;
                                 passed &= passed - 1;
                                 float4 h = queue.result[b];
+                                const uint32_t ti = queue.pair[b].x;
                                 if (LEAF == GZG_LEAF_WATERTIGHT) {
                                         // its limit is rounded with the triangle's
                                         // determinant: tested again against the
                                         // hits before it
-                                        const uint32_t ti = queue.pair[b].x;
                                         if (!leaf_test<LEAF>(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, __ldg(s.tv0 + ti),
                                                              __ldg(s.tv1 + ti), __ldg(s.tv2 + ti), thit, h.x, h.y, h.z))
                                                 continue;
                                 } else if (h.x > thit) {  // as mt_test: a NaN limit or distance accepts
                                         continue;
+                                }
+                                if (!ANY && !(h.x <= thit && (prim < 0 || box_before(s, r, ti, h.x))) &&
+                                    !(r.oct & kAlone)) {
+                                        again = true;
+                                        break;
                                 }
                                 thit = h.x;
                                 bu = h.y;
@@ -703,7 +752,17 @@ __global__ void __launch_bounds__(128, 8) k_wide_queued(DevScene s, const void *
                         __syncwarp();
                         mine = 0u;
                         queued = 0u;
-                        if (ANY) have = __ballot_sync(FULL, tris != 0u);
+                        if (again) {
+                                const RayIn in = load_ray<RAYFMT>(rays, tmaxs, ray_i);
+                                thit = in.tmax;
+                                prim = -1;
+                                sp = 0;
+                                steps = 0;
+                                group = make_uint2(s.per_ray_root ? in.root : 0u, (1u << 24) | (1u << r.oct));
+                                r.oct |= kAlone;
+                                tris = 0u;
+                        }
+                        have = __ballot_sync(FULL, tris != 0u);
                 }
                 if (ray_i >= 0 && mine == 0u && (ANY ? prim >= 0 || (group.y >> 24) == 0u : (group.y >> 24) == 0u)) {
                         if (prim < 0) {
@@ -957,8 +1016,10 @@ constexpr int kQueueTestsInst = 12, kQueueWaitingInst = 4;
 // leaves hold instances only and the bottom levels' triangles only, so an
 // instance is entered where its record is met and triangles are queued; a ray
 // whose triangles are still queued waits before it leaves its instance, because
-// they are tested with its object-space ray.  2M rays through 4096 instances
-// 1,359 -> 1,215 us, two-level frame 26.2 -> 24.4 ms.
+// they are tested with its object-space ray (so top-level nodes are always opened
+// with the nearest hit known, and starting over is decided by the instance's own
+// boxes).  2M rays through 4096 instances
+// 1,359 -> 1,219 us, two-level frame 26.2 -> 24.6 ms.
 template <int OUTFMT, bool ANY, int STACK>
 __global__ void __launch_bounds__(128, 8) k_wide_instanced_queued(DevScene s, const void *__restrict__ rays,
                                                                   const float *__restrict__ tmaxs, int64_t n,
@@ -973,13 +1034,13 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced_queued(DevScene s, co
 
         uint2 *stack = smem_stack + threadIdx.x;
         const int stride = blockDim.x;
-        TriQueue &queue = reinterpret_cast<TriQueue *>(smem_stack + STACK * blockDim.x)[threadIdx.x >> 5];
+        InstQueue &queue = reinterpret_cast<InstQueue *>(smem_stack + STACK * blockDim.x)[threadIdx.x >> 5];
         uint32_t queued = 0;  // pairs in the queue (warp-uniform)
         uint32_t mine = 0;    // queue positions of this lane's ray
         int ray_i = -1;
         WideRay r;
-        float thit = 0.0f, bu = 0.0f, bv = 0.0f;
-        int prim = -1, hit_inst = -1, cur_inst = -1, sp = 0;
+        float thit = 0.0f;
+        int prim = -1, cur_inst = -1, sp = 0;
         uint2 group = make_uint2(0u, 0u);
         uint32_t steps = 0;
 
@@ -1001,8 +1062,7 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced_queued(DevScene s, co
                                 r.dz = in.dz;
                                 set_ray_dirs(r, s.rcp_max);
                                 thit = in.tmax;
-                                bu = bv = 0.0f;
-                                prim = hit_inst = cur_inst = -1;
+                                prim = cur_inst = -1;
                                 sp = 0;
                                 steps = 0;
                                 group = make_uint2(0u, (1u << 24) | (1u << r.oct));
@@ -1030,7 +1090,9 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced_queued(DevScene s, co
                                 }
                                 --sp;
                                 world_ray(rays, ray_i, r);
+                                const uint32_t alone = r.oct & kAlone;
                                 set_ray_dirs(r, s.rcp_max);
+                                r.oct |= alone;
                                 cur_inst = -1;
                         } else {
                                 --sp;
@@ -1048,7 +1110,7 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced_queued(DevScene s, co
                         const uint32_t key = __ffs(hits) - 1;
                         hits &= hits - 1;
                         const uint32_t im = group.y & 0xFFu;
-                        const uint32_t slot = key ^ r.oct;
+                        const uint32_t slot = (key ^ r.oct) & 7u;
                         const uint32_t node = group.x + __popc(im & ((1u << slot) - 1u));
                         if (hits) {
                                 if (sp >= STACK) {
@@ -1117,9 +1179,11 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced_queued(DevScene s, co
                                 r.dx = xf_vector(m0, w.dx, w.dy, w.dz);
                                 r.dy = xf_vector(m1, w.dx, w.dy, w.dz);
                                 r.dz = xf_vector(m2, w.dx, w.dy, w.dz);
+                                const uint32_t alone = r.oct & kAlone;
                                 set_ray_dirs(r, s.rcp_max);
                                 cur_inst = inst;
                                 group = make_uint2((uint32_t)__float_as_int(m3.x), (1u << 24) | (1u << r.oct));
+                                r.oct |= alone;
                         }
                 }
                 if (fault) {
@@ -1134,25 +1198,32 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced_queued(DevScene s, co
                 unsigned have = __ballot_sync(FULL, tris != 0u);
                 while ((have | queued) != 0u) {
                         if (have != 0u) {
-                                queued = queue_append(queue, queued, have, tris, tri_base, tri_bits, mine);
+                                queued = queue_append(queue, queued, have, tris, tri_base, tri_bits, mine,
+                                                      !ANY && (r.oct & kAlone) ? 1 : 7);
                                 have = __ballot_sync(FULL, tris != 0u);  // what found no room
                         }
-                        if (have == 0u && queued < kQueueTestsInst) {
+                        if (have == 0u && queued < kQueueTestsInst &&
+                            (ANY || !__any_sync(FULL, (r.oct & kAlone) && mine != 0u))) {
                                 const unsigned waiting = __ballot_sync(FULL, waits);
                                 const unsigned busy = __ballot_sync(FULL, ray_i >= 0 && !waits);
                                 if (busy != 0u && __popc(waiting) < kQueueWaitingInst) break;
                         }
+                        bool again = false;
                         uint32_t passed = queue_test<GZG_LEAF_MOLLER_TRUMBORE>(s, queue, queued, r, thit) & mine;
                         while (passed) {
                                 const uint32_t b = __ffs(passed) - 1;
                                 passed &= passed - 1;
                                 const float4 h = queue.result[b];
                                 if (h.x > thit) continue;  // as mt_test: a NaN limit or distance accepts
+                                if (!ANY && !(h.x <= thit && (prim < 0 || box_before(s, r, queue.pair[b].x, h.x))) &&
+                                    !(r.oct & kAlone)) {
+                                        again = true;
+                                        break;
+                                }
                                 thit = h.x;
-                                bu = h.y;
-                                bv = h.z;
+                                queue.uv[lane] = make_float2(h.y, h.z);
                                 prim = __float_as_int(h.w);
-                                hit_inst = cur_inst;
+                                queue.inst[lane] = cur_inst;
                                 if (ANY) {
                                         tris = 0u;
                                         break;
@@ -1161,17 +1232,27 @@ __global__ void __launch_bounds__(128, 8) k_wide_instanced_queued(DevScene s, co
                         __syncwarp();
                         mine = 0u;
                         queued = 0u;
-                        if (ANY) have = __ballot_sync(FULL, tris != 0u);
+                        if (again) {
+                                thit = load_ray<kRayDevice>(rays, tmaxs, ray_i).tmax;
+                                world_ray(rays, ray_i, r);
+                                set_ray_dirs(r, s.rcp_max);
+                                prim = cur_inst = -1;
+                                sp = 0;
+                                steps = 0;
+                                group = make_uint2(0u, (1u << 24) | (1u << r.oct));
+                                r.oct |= kAlone;
+                                tris = 0u;
+                                waits = false;
+                        }
+                        have = __ballot_sync(FULL, tris != 0u);
                 }
                 if (ray_i >= 0 && mine == 0u && ((ANY && prim >= 0) || ((group.y >> 24) == 0u && sp == 0))) {
                         if (prim < 0) {
                                 thit = load_ray<kRayDevice>(rays, tmaxs, ray_i).tmax;
-                                bu = 0.0f;
-                                bv = 0.0f;
-                                hit_inst = -1;
                         }
-                        store_hit<OUTFMT>(s, out, ray_i, prim, thit, bu, bv);
-                        if (s.inst_out) s.inst_out[ray_i] = hit_inst;
+                        const float2 uv = prim < 0 ? make_float2(0.0f, 0.0f) : queue.uv[lane];
+                        store_hit<OUTFMT>(s, out, ray_i, prim, thit, uv.x, uv.y);
+                        if (s.inst_out) s.inst_out[ray_i] = prim < 0 ? -1 : queue.inst[lane];
                         ray_i = -1;
                         group.y = 0u;
                         sp = 0;
@@ -1320,7 +1401,7 @@ cudaError_t launch_wide_kernel(TraceKernel k, int stack, bool persistent, bool q
         // (measured faster for any-hit queries than a 256-thread bound).
         const int block = (p.block_size == 64 || (p.block_size == 256 && !persistent)) ? p.block_size : 128;
         const int blocks_per_sm = p.blocks_per_sm;
-        const size_t smem = (size_t)stack * block * sizeof(uint2) + (queued ? (size_t)(block / 32) * sizeof(TriQueue) : 0);
+        const size_t smem = (size_t)stack * block * sizeof(uint2) + (queued ? (size_t)(block / 32) * (s.instances ? sizeof(InstQueue) : sizeof(TriQueue)) : 0);
         if (smem > 48 * 1024) {
                 cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 if (e != cudaSuccess) return e;

@@ -165,3 +165,101 @@ def test_two_level_nan_limit_gives_one_answer():
         assert torch.equal(inst[0], inst[1]) and bool((inst[0][::3] >= 0).any())
     for b in blas:
         b.close()
+
+
+def _slivers(rng, count):
+    """Needles in the plane y = 0, on top of one another: a ray meets several
+    at the same distance, which their tests compute with relative errors of
+    1e-7 to 1e-4, well past a box's slack."""
+    sb = scenes.SceneBuilder()
+    m = sb.add_material()
+    c, a = rng.uniform(0, 1, (count, 2)), rng.uniform(0, 2 * np.pi, count)
+    along = 0.5 * np.stack([np.cos(a), np.sin(a)], 1)
+    across = rng.uniform(2e-4, 2e-2, (count, 1)) * np.stack([-np.sin(a), np.cos(a)], 1)
+    p = np.stack([c - along, c + along, c + across], 1).reshape(-1, 2)
+    pts = np.stack([p[:, 0], np.zeros(len(p)), p[:, 1]], 1).astype(np.float32)
+    sb.add_mesh(pts, np.arange(3 * count).reshape(-1, 3), m)
+    return sb.build()
+
+
+def _grazing_rays(rng, n):
+    target = np.stack([rng.uniform(0, 1, n), np.zeros(n), rng.uniform(0, 1, n)], 1)
+    a, e = rng.uniform(0, 2 * np.pi, n), 10.0 ** rng.uniform(-2, 0, n)
+    d = np.stack([np.cos(a), -e, np.sin(a)], 1)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o = target - d * 10.0 ** rng.uniform(0, 1.5, (n, 1))
+    rays = scenes.pack_device_rays(o.astype(np.float32), d.astype(np.float32), np.full(n, np.inf, np.float32))
+    rays[::1000, 5] = np.nan  # a direction with a NaN: every distance is one
+    return rays
+
+
+@pytest.mark.parametrize("leaf", [F.LEAF_MOLLER_TRUMBORE, F.LEAF_WATERTIGHT])
+def test_a_rays_hit_depends_on_the_ray_alone(leaf):
+    """Triangles whose computed distance falls before their own box: which
+    nodes a ray has opened before its queued triangles are tested must not
+    decide its hit.  The one-ray-per-thread kernel prunes at once."""
+    import torch
+
+    rng = np.random.default_rng(21)
+    with GpuAccelerator(_slivers(rng, 4000)) as acc:
+        n = 390 * acc.info()["wide_nodes"]
+        rays = torch.from_numpy(_grazing_rays(rng, n)).cuda()
+        order = torch.from_numpy(rng.permutation(n)).cuda()
+        one, got, mixed = (torch.empty((n, 4), device="cuda") for _ in range(3))
+        acc.trace_closest(rays, one, options(leaf_test=leaf, traversal=F.TRAVERSAL_WIDE_ONE_RAY_PER_THREAD))
+        acc.trace_closest(rays, got, options(leaf_test=leaf))
+        acc.trace_closest(rays[order].contiguous(), mixed, options(leaf_test=leaf))
+        torch.cuda.synchronize()
+        bits = one.view(torch.int32)
+        assert int((got.view(torch.int32) != bits).any(1).sum()) == 0
+        assert int((mixed.view(torch.int32) != bits[order]).any(1).sum()) == 0
+        assert bool((bits[:, 3] >= 0).any()) and acc.error_word() == 0
+
+
+def test_two_level_hit_depends_on_the_ray_alone():
+    import torch
+
+    rng = np.random.default_rng(22)
+    blas = [GpuAccelerator(_slivers(rng, 1000)) for _ in range(2)]
+    with InstancedAccelerator(blas, scenes.random_instances(6, 2, 5, extent=0.3)) as acc:
+        n = 400 * acc.info()["wide_nodes"] + 555
+        rays = torch.from_numpy(_grazing_rays(rng, n)).cuda()
+        whole, w_inst = torch.empty((n, 4), device="cuda"), torch.empty(n, dtype=torch.int32, device="cuda")
+        got, g_inst = torch.empty_like(whole), torch.empty_like(w_inst)
+        acc.trace_closest(rays, whole, w_inst)
+        for s in _slices(n, 1 + n // 5):
+            acc.trace_closest(rays[s], got[s], g_inst[s])
+        torch.cuda.synchronize()
+        bad = (got.view(torch.int32) != whole.view(torch.int32)).any(1) | (g_inst != w_inst)
+        assert int(bad.sum()) == 0
+        assert bool((w_inst >= 0).any()) and acc.error_word() == 0
+    for b in blas:
+        b.close()
+
+
+@pytest.mark.parametrize("leaf", [F.LEAF_MOLLER_TRUMBORE, F.LEAF_WATERTIGHT])
+def test_dense_sphere_hits_depend_on_the_ray_alone(leaf):
+    """Rays at the vertices and edges of a dense sphere and along its surface."""
+    import torch
+
+    pts, tris = scenes.displaced_icosphere(7, seed=3)
+    sb = scenes.SceneBuilder()
+    sb.add_mesh(pts, tris, sb.add_material())
+    rng = np.random.default_rng(23)
+    n = 2_000_000
+    pick = tris[rng.integers(0, len(tris), n)]
+    s = rng.uniform(0, 1, (n, 1)) * (rng.random((n, 1)) < 0.7)  # the rest at a vertex
+    target = (1 - s) * pts[pick[:, 0]] + s * pts[pick[:, 1]]
+    out = target / np.linalg.norm(target, axis=1, keepdims=True)
+    d = rng.normal(size=(n, 3))
+    d -= out * (d * out).sum(1, keepdims=True) * rng.choice([0.0, 0.97, 1.0], (n, 1))  # a third tangent, a third nearly
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o = (target - 3.0 * d).astype(np.float32)
+    with GpuAccelerator(sb.build()) as acc:
+        rays = torch.from_numpy(scenes.pack_device_rays(o, d.astype(np.float32), np.full(n, np.inf, np.float32))).cuda()
+        one, got = torch.empty((n, 4), device="cuda"), torch.empty((n, 4), device="cuda")
+        acc.trace_closest(rays, one, options(leaf_test=leaf, traversal=F.TRAVERSAL_WIDE_ONE_RAY_PER_THREAD))
+        acc.trace_closest(rays, got, options(leaf_test=leaf))
+        torch.cuda.synchronize()
+        assert int((got.view(torch.int32) != one.view(torch.int32)).any(1).sum()) == 0
+        assert bool((one[:, 3].view(torch.int32) >= 0).any())
