@@ -447,7 +447,9 @@ gzg_status host_batch(gzg_scene *s, const gzg_ray *rays, const float *tmax, int6
                                 }
                                 if (ws) message[k] = g_last_error;
                         } catch (const std::exception &) {
-                                ws = GZG_ERR_OUT_OF_MEMORY;
+                                // (a chunk whose wait ran out is still in flight,
+                                // whatever failed after it)
+                                if (ws != GZG_ERR_TIMEOUT) ws = GZG_ERR_OUT_OF_MEMORY;
                         }
                         if (ws) stop = true;
                         status[k] = ws;
@@ -477,7 +479,9 @@ gzg_status host_batch(gzg_scene *s, const gzg_ray *rays, const float *tmax, int6
                 for (int pass = 0; pass < 2 && !st; ++pass)
                         for (int k = 0; k <= helpers && !st; ++k)
                                 if (status[k] && (pass == 1 || status[k] == GZG_ERR_TIMEOUT))
-                                        st = set_error(status[k], message[k].empty() ? "batch call: out of host memory" : message[k]);
+                                        st = set_error(status[k], !message[k].empty()                ? message[k]
+                                                                  : status[k] == GZG_ERR_TIMEOUT ? "batch chunk: no completion in time"
+                                                                                                 : "batch call: out of host memory");
         }
         if (st != GZG_OK) {
                 // A wait that ran out leaves chunks in flight on the staging

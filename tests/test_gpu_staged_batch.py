@@ -2,12 +2,13 @@
 chunks, against the same call on pinned arrays (one thread, copied directly):
 the same bytes at counts around the chunk sizes, for every result format, with
 callers running at once, and a time-out that leaves the scene usable."""
+import os
 import threading
 
 import numpy as np
 import pytest
 
-from gonzales_b200 import GpuAccelerator, scenes
+from gonzales_b200 import GpuAccelerator, GzgError, scenes
 from gonzales_b200 import _ffi as F
 
 pytestmark = pytest.mark.gpu
@@ -65,3 +66,33 @@ def test_callers_at_once(rays):
         th.join()
     for k in range(6):
         assert got[k].tobytes() == ref[k * 1000:].tobytes()
+
+
+GZG_ERR_TIMEOUT = 8
+
+
+def test_time_out_of_a_staged_call(rays, monkeypatch):
+    """Every worker's wait runs out (on the host: 1 us), its chunk still in
+    flight: the caller gets the time-out and its message, the slots' buffers are
+    left to their chunks, every helper thread has ended, and the next calls are
+    served as before, also while those chunks still run."""
+    import torch
+
+    acc, r6, t = rays
+    n = 1_000_000
+    ref = acc.intersect_batch(r6[:n], t[:n])
+    threads = len(os.listdir("/proc/self/task"))
+    for k in range(4):
+        monkeypatch.setenv("GZG_WAIT_LIMIT_US", "1")
+        with pytest.raises(GzgError) as e:
+            acc.intersect_batch(r6[:n], t[:n])
+        assert e.value.status == GZG_ERR_TIMEOUT and "GZG_WAIT_LIMIT_US" in str(e.value)
+        monkeypatch.delenv("GZG_WAIT_LIMIT_US")
+        if k % 2 == 0:
+            torch.cuda.synchronize()  # the abandoned chunks have run
+        again = acc.intersect_batch(r6[:n], t[:n])
+        assert again.tobytes() == ref.tobytes()
+        assert acc.error_word() == 0
+    assert len(os.listdir("/proc/self/task")) == threads
+    torch.cuda.synchronize()
+    assert acc.occluded_batch(r6[:n], t[:n]).sum() == (ref["hit"] != 0).sum()
