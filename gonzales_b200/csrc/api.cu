@@ -7,11 +7,13 @@
 #include <atomic>
 #include <array>
 #include <cmath>
+#include <condition_variable>
 #include <cstring>
 #include <memory>
 #include <chrono>
 #include <cstdlib>
 #include <mutex>
+#include <optional>
 #include <thread>
 #include <string>
 #include <vector>
@@ -63,12 +65,12 @@ class DeviceGuard {
         int prev_ = 0, dev_ = 0;
 };
 
-constexpr int kSlots = 8;             // chunks in flight of one staged call
-constexpr int kDirectSlots = 4;       // of one that copies from and to pinned host arrays
-constexpr int64_t kChunk = 1 << 19;   // rays per chunk of pinned arrays (512K x 4 streams: 2 % faster end to end than 1M x 3)
-// Staged chunks are small, so that the copies in, the transfers, the trace and
-// the copies out of one call overlap, but no smaller than what a copy's and a
-// launch's overhead is worth.
+constexpr int kSlots = 8;             // threads of one staged call, each with a chunk in flight
+constexpr int kOneThreadSlots = 4;    // chunks in flight of a call that one thread serves
+constexpr int64_t kChunk = 1 << 19;   // and their rays (pinned arrays: 512K x 4 streams 2 % faster end to end than 1M x 3)
+// The chunks of several threads are small, so that the copies in, the transfers,
+// the trace and the copies out of one call overlap, but no smaller than what a
+// copy's and a launch's overhead is worth.
 constexpr int64_t kStagedChunkMin = 1 << 14, kStagedChunkMax = 1 << 17;
 
 // Per-call staging: device buffers, and pinned host buffers for pageable
@@ -128,9 +130,73 @@ struct Staging {
         }
 };
 
-// Helper threads of staged calls running now, over all scenes and callers:
-// callers that already keep every core busy get none.
-std::atomic<int> g_helpers{0};
+// Who makes staged calls, over all scenes: a call has the process to itself when
+// none else is running and the one before it came from the same thread.  Callers
+// that take turns or overlap keep the cores busy by themselves.
+std::atomic<int> g_staged_calls{0};
+std::atomic<const void *> g_staged_caller{nullptr};
+struct StagedCall {
+        static const void *self() {
+                static thread_local char here;
+                return &here;
+        }
+        const bool first = g_staged_calls.fetch_add(1) == 0;
+        const void *const before = g_staged_caller.exchange(self());
+        const bool alone = first && (before == nullptr || before == self());
+        StagedCall() = default;
+        StagedCall(const StagedCall &) = delete;
+        ~StagedCall() { g_staged_calls.fetch_sub(1); }
+};
+
+// Microseconds a host wait may take (0: no limit).
+int64_t wait_limit_us() {
+        const char *env = std::getenv("GZG_WAIT_LIMIT_US");
+        return env ? std::atoll(env) : 300000000;
+}
+gzg_status timed_out(const char *what, int64_t limit_us) {
+        return set_error(GZG_ERR_TIMEOUT, std::string(what) + ": no completion within " + std::to_string(limit_us) +
+                                              " us (GZG_WAIT_LIMIT_US)");
+}
+
+// Calls of up to kTurnRays rays that one thread serves take turns, kTurns at
+// once: they are mostly driver calls, and beyond ten threads making those at once
+// each slows the others (16,000 pageable rays a call on 16 cores: 8 callers 245
+// Mrays/s, 10 the same, 12 195, 15 125; with turns 250 at 15 and 30).  Larger calls are
+// mostly copies, which every core helps with.
+constexpr int kTurns = 8;
+constexpr int64_t kTurnRays = 1 << 17;
+class Turn {
+    public:
+        Turn() = default;
+        Turn(const Turn &) = delete;
+        ~Turn() {
+                if (!held_) return;
+                {
+                        std::lock_guard<std::mutex> lk(mu_);
+                        ++free_;
+                }
+                cv_.notify_one();
+        }
+        gzg_status take() {
+                std::unique_lock<std::mutex> lk(mu_);
+                const int64_t limit = wait_limit_us();
+                auto ready = [] { return free_ > 0; };
+                if (limit <= 0) {
+                        cv_.wait(lk, ready);
+                } else if (!cv_.wait_for(lk, std::chrono::microseconds(limit), ready)) {
+                        return timed_out("batch turn", limit);
+                }
+                --free_;
+                held_ = true;
+                return GZG_OK;
+        }
+
+    private:
+        bool held_ = false;
+        static inline std::mutex mu_;
+        static inline std::condition_variable cv_;
+        static inline int free_ = kTurns;
+};
 
 bool is_pinned(const void *p) {
         cudaPointerAttributes a;
@@ -201,12 +267,12 @@ struct gzg_scene {
         // host copies of the shading arrays (batch assembly)
         HostShading host_shading;
         std::mutex pool_mu;
-        std::vector<std::unique_ptr<Staging>> pool;
+        std::vector<std::unique_ptr<Staging>> pool[2];  // of calls one thread serves, and of several
         PullRing pull;
 
         ~gzg_scene() {
                 DeviceGuard g(device);
-                pool.clear();
+                for (auto &p : pool) p.clear();
                 pull.release();
                 for (void *p : allocs) cudaFree(p);
         }
@@ -235,12 +301,15 @@ struct gzg_scene {
                 return GZG_OK;
         }
 
-        gzg_status acquire(std::unique_ptr<Staging> *out) {
+        // (Calls of several threads and of one have pools of their own: their
+        // chunks differ in size, and buffers are not made again for either.)
+        gzg_status acquire(std::unique_ptr<Staging> *out, bool threads) {
                 {
                         std::lock_guard<std::mutex> lk(pool_mu);
-                        if (!pool.empty()) {
-                                *out = std::move(pool.back());
-                                pool.pop_back();
+                        auto &free = pool[threads];
+                        if (!free.empty()) {
+                                *out = std::move(free.back());
+                                free.pop_back();
                                 return GZG_OK;
                         }
                 }
@@ -249,15 +318,14 @@ struct gzg_scene {
                 *out = std::move(s);
                 return GZG_OK;
         }
-        void release(std::unique_ptr<Staging> s) {
+        void release(std::unique_ptr<Staging> s, bool threads) {
                 std::lock_guard<std::mutex> lk(pool_mu);
-                pool.push_back(std::move(s));
+                pool[threads].push_back(std::move(s));
         }
 };
 
 gzg_status gzg::wait_stream(void *stream, const char *what) {
-        int64_t limit_us = 300000000;
-        if (const char *env = std::getenv("GZG_WAIT_LIMIT_US")) limit_us = std::atoll(env);
+        const int64_t limit_us = wait_limit_us();
         cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
         cudaEvent_t ev = nullptr;
         cudaError_t e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
@@ -278,8 +346,7 @@ gzg_status gzg::wait_stream(void *stream, const char *what) {
                 const int64_t us =
                     std::chrono::duration_cast<std::chrono::microseconds>(std::chrono::steady_clock::now() - t0).count();
                 if (limit_us > 0 && us >= limit_us) {
-                        status = set_error(GZG_ERR_TIMEOUT, std::string(what) + ": no completion within " +
-                                                                std::to_string(limit_us) + " us (GZG_WAIT_LIMIT_US)");
+                        status = timed_out(what, limit_us);
                         break;
                 }
                 // spin with yields for the first 2 ms (batch chunks finish in
@@ -376,8 +443,12 @@ cudaError_t device_trace(gzg_scene *scene, LaunchParams p, int out_fmt, const vo
 // `out_bytes` per ray in format `out_fmt`.  Pinned arrays are copied from and to
 // directly.  Pageable ones go through the pinned staging buffers, and there the
 // host's copies are what the call waits for (76 bytes a ray through one core:
-// 1M rays took 9.0 ms, of which 1.4 ms PCIe and 0.3 ms tracing), so several
-// threads each take chunks through a slot of their own.
+// 1M rays took 9.0 ms, of which 1.4 ms PCIe and 0.3 ms tracing).  A staged call
+// that has the process to itself takes several threads, each with chunks through
+// a slot of its own (2.4 ms).  Of several callers (a tile renderer's tasks) each
+// stages on its own thread, with kOneThreadSlots chunks in flight: 15 callers on
+// 16 cores with 300,000 rays each got 190 to 370 Mrays/s when every call could
+// take helper threads, and get 540 to 600.
 gzg_status host_batch(gzg_scene *s, const gzg_ray *rays, const float *tmax, int64_t count, void *results,
                       size_t out_bytes, int out_fmt, const gzg_trace_options *opt) {
         if (!s || count < 0 || (count > 0 && (!rays || !tmax || !results)))
@@ -389,19 +460,27 @@ gzg_status host_batch(gzg_scene *s, const gzg_ray *rays, const float *tmax, int6
         if (st != GZG_OK) return st;
         if (count == 0) return clear_error();
         DeviceGuard g(s->device);
-        std::unique_ptr<Staging> stg;
-        st = s->acquire(&stg);
-        if (st != GZG_OK) return st;
         const LaunchParams base = params_for(s, opt, out_fmt == kOutAnyPrim || out_fmt == kOutOccluded);
         const bool direct = is_pinned(rays) && is_pinned(tmax) && is_pinned(results);
+        std::optional<StagedCall> staged;
+        if (!direct) staged.emplace();
+        int threads = 1;
+        if (staged && staged->alone && count > kStagedChunkMin)
+                threads = std::min(kSlots, (int)std::max(1u, std::thread::hardware_concurrency()));
+        Turn turn;
+        if (threads == 1 && count <= kTurnRays && (st = turn.take())) return st;
+        std::unique_ptr<Staging> stg;
+        st = s->acquire(&stg, threads > 1);
+        if (st != GZG_OK) return st;
         int64_t chunk = kChunk;
-        if (!direct) {
-                // two chunks a slot or more, a power of two so that slots keep few sizes
+        if (threads > 1) {
+                // one to two chunks a thread between the limits, a power of two
+                // so that slots keep few sizes
                 chunk = kStagedChunkMin;
                 while (chunk < kStagedChunkMax && chunk * 2 * kSlots < count) chunk *= 2;
         }
         const int64_t nchunks = (count + chunk - 1) / chunk;
-        const int slots = (int)std::min<int64_t>(direct ? kDirectSlots : kSlots, nchunks);
+        const int slots = (int)std::min<int64_t>(threads > 1 ? threads : kOneThreadSlots, nchunks);
         char *res = reinterpret_cast<char *>(results);
         auto enqueue = [&](int k, int64_t c) -> gzg_status {
                 Staging::Slot &q = stg->slot[k];
@@ -422,10 +501,32 @@ gzg_status host_batch(gzg_scene *s, const gzg_ray *rays, const float *tmax, int6
                        "result download");
                 return GZG_OK;
         };
-        if (direct) {
-                for (int k = 0; k < slots && !st; ++k) st = stg->ensure(k, chunk, false);
-                for (int64_t c = 0; c < nchunks && !st; ++c) st = enqueue((int)(c % slots), c);
-                for (int k = 0; k < slots && !st; ++k) st = wait_stream(stg->slot[k].st, "batch sync");
+        if (threads == 1) {
+                const int64_t room = count <= kStagedChunkMin ? kStagedChunkMin : kChunk;
+                auto drain = [&](int64_t c) -> gzg_status {
+                        Staging::Slot &q = stg->slot[c % slots];
+                        const gzg_status ws = wait_stream(q.st, direct ? "batch sync" : "batch chunk");
+                        if (ws || direct) return ws;
+                        const int64_t off = c * chunk, n = std::min(chunk, count - off);
+                        std::memcpy(res + off * out_bytes, q.h_out, (size_t)n * out_bytes);
+                        return GZG_OK;
+                };
+                for (int64_t c = 0; c < nchunks && !st; ++c) {
+                        const int k = (int)(c % slots);
+                        if (c < slots) {
+                                st = stg->ensure(k, room, !direct);
+                        } else if (!direct) {
+                                st = drain(c - slots);
+                        }
+                        if (st) break;
+                        if (!direct) {
+                                const int64_t off = c * chunk, n = std::min(chunk, count - off);
+                                std::memcpy(stg->slot[k].h_in, rays + off, (size_t)n * sizeof(gzg_ray));
+                                std::memcpy(stg->slot[k].h_tmax, tmax + off, (size_t)n * sizeof(float));
+                        }
+                        st = enqueue(k, c);
+                }
+                for (int64_t c = nchunks - slots; c < nchunks && !st; ++c) st = drain(c);
         } else {
                 std::atomic<int64_t> next{0};
                 std::atomic<bool> stop{false};
@@ -454,26 +555,16 @@ gzg_status host_batch(gzg_scene *s, const gzg_ray *rays, const float *tmax, int6
                         if (ws) stop = true;
                         status[k] = ws;
                 };
-                // helpers beside the calling thread, as far as the cores go
+                // helpers beside the calling thread
                 int helpers = 0;
                 std::thread helper[kSlots];
-                const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
-                while (helpers + 1 < slots) {
-                        if (g_helpers.fetch_add(1) + 1 >= cores) {
-                                g_helpers.fetch_sub(1);
-                                break;
-                        }
-                        try {
-                                helper[helpers] = std::thread(work, helpers + 1);
-                        } catch (const std::exception &) {
-                                g_helpers.fetch_sub(1);
-                                break;
-                        }
-                        ++helpers;
+                try {
+                        for (; helpers + 1 < slots; ++helpers) helper[helpers] = std::thread(work, helpers + 1);
+                } catch (const std::exception &) {
+                        // (as many as the system allows)
                 }
                 work(0);
                 for (int k = 0; k < helpers; ++k) helper[k].join();
-                g_helpers.fetch_sub(helpers);
                 // a wait that ran out comes before any other failure: its
                 // chunk is still in flight
                 for (int pass = 0; pass < 2 && !st; ++pass)
@@ -490,7 +581,7 @@ gzg_status host_batch(gzg_scene *s, const gzg_ray *rays, const float *tmax, int6
                 if (st == GZG_ERR_TIMEOUT) stg.release();
                 return st;
         }
-        s->release(std::move(stg));
+        s->release(std::move(stg), threads > 1);
         uint32_t w = 0;
         st = read_error_word(s, &w, true);
         if (st != GZG_OK) return st;

@@ -96,3 +96,36 @@ def test_time_out_of_a_staged_call(rays, monkeypatch):
     assert len(os.listdir("/proc/self/task")) == threads
     torch.cuda.synchronize()
     assert acc.occluded_batch(r6[:n], t[:n]).sum() == (ref["hit"] != 0).sum()
+
+
+def test_callers_at_once_take_no_helpers(rays):
+    """A call that runs by itself may take 7 helper threads; callers that run at
+    the same time stage on their own threads (a chunk ring that wraps here), and
+    give the same bytes."""
+    acc, r6, t = rays
+    r6, t = np.tile(r6, (3, 1)), np.tile(t, 3)
+    ref = _direct(acc, r6, t)
+    base, most, got = len(os.listdir("/proc/self/task")), [0], [None] * 8
+    start = threading.Barrier(8)
+
+    def call(k):
+        start.wait()
+        n = len(t) - 7777 * k if k < 3 else 300_000 + k  # over and under the ring's chunks
+        for _ in range(1 if k < 3 else 6):
+            got[k] = acc.intersect_batch(r6[:n], t[:n])
+            most[0] = max(most[0], len(os.listdir("/proc/self/task")))
+
+    def watch():
+        while any(th.is_alive() for th in threads):
+            most[0] = max(most[0], len(os.listdir("/proc/self/task")))
+
+    threads = [threading.Thread(target=call, args=(k,)) for k in range(8)]
+    for th in threads:
+        th.start()
+    watch()
+    for th in threads:
+        th.join()
+    for k in range(8):
+        assert got[k].tobytes() == ref[:len(got[k])].tobytes()
+    assert most[0] <= base + 8 + 7, "more helpers than one call's"
+    assert acc.error_word() == 0
