@@ -1752,6 +1752,18 @@ __global__ void k_zsobol_fill(ZSobolConfig c, const int32_t *px, const int32_t *
         }
 }
 
+// The nibble tables (sobol.cuh) from the matrices, one word per thread.
+__global__ void k_sobol_nibbles(const uint32_t *matrices, uint32_t *nibbles) {
+        const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;  // [dim][8 groups][16 values]
+        const uint32_t *m = matrices + (size_t)(i / kSobolNibbleWords) * kSobolColumns + 4 * ((i >> 4) & 7u);
+        uint32_t x = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+                if ((i >> b) & 1u) x ^= m[b];
+        nibbles[i] = x;
+}
+static_assert(kSobolDims * kSobolNibbleWords % 256 == 0, "k_sobol_nibbles fills whole blocks");
+
 // ------------------------------------------------------------ host side
 
 std::mutex g_sobol_mu;
@@ -1765,23 +1777,24 @@ gzg_status device_sobol(int dev, const uint32_t **out) {
                 const uint32_t *host = sobol_matrices(&count);
                 if (count != (size_t)kSobolDims * kSobolColumns)
                         return set_error(GZG_ERR_BAD_SCENE, "embedded Sobol table has the wrong size");
-                // the matrices, then the nibble tables made from them
-                std::vector<uint32_t> table(host, host + count);
-                table.resize(count + (size_t)kSobolDims * kSobolNibbleWords);
-                for (int d = 0; d < kSobolDims; ++d)
-                        for (int g = 0; g < 8; ++g)
-                                for (int v = 0; v < 16; ++v) {
-                                        uint32_t x = 0;
-                                        for (int b = 0; b < 4; ++b)
-                                                if ((v >> b) & 1) x ^= host[(size_t)d * kSobolColumns + 4 * g + b];
-                                        table[count + (size_t)d * kSobolNibbleWords + 16 * g + v] = x;
-                                }
-                void *p = nullptr;
-                cudaError_t e = cudaMalloc(&p, table.size() * 4);
+                // the matrices, then the nibble tables made from them on the
+                // device (on one host core: 0.4 ms of a process's first renderer)
+                constexpr size_t nibbles = (size_t)kSobolDims * kSobolNibbleWords;
+                uint32_t *p = nullptr;
+                cudaError_t e = cudaMalloc(&p, (count + nibbles) * 4);
                 if (e != cudaSuccess) return set_error(GZG_ERR_OUT_OF_MEMORY, "Sobol table allocation");
-                e = cudaMemcpy(p, table.data(), table.size() * 4, cudaMemcpyHostToDevice);
-                if (e != cudaSuccess) return set_error(GZG_ERR_CUDA, "Sobol table upload");
-                g_sobol_dev[dev] = static_cast<const uint32_t *>(p);
+                const cudaStream_t st = cudaStreamPerThread;
+                e = cudaMemcpyAsync(p, host, count * 4, cudaMemcpyHostToDevice, st);
+                if (e == cudaSuccess) {
+                        k_sobol_nibbles<<<nibbles / 256, 256, 0, st>>>(p, p + count);
+                        e = cudaGetLastError();
+                }
+                if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+                if (e != cudaSuccess) {
+                        cudaFree(p);
+                        return set_error(GZG_ERR_CUDA, "Sobol table upload");
+                }
+                g_sobol_dev[dev] = p;
         }
         *out = g_sobol_dev[dev];
         return GZG_OK;

@@ -26,3 +26,14 @@ def test_sampler_bits_at_index_widths(spp, res, seed):
     ours = device_zsobol(spp, res[0], res[1], px, py, idx, kinds, seed=seed)
     ref = O.zsobol_batch(spp, res[0], res[1], px, py, idx, kinds, seed=seed)
     assert ours.tobytes() == ref.tobytes()
+
+
+def test_nibble_tables_of_many_dimensions():
+    """The tables that the device fills from the matrices: 192 dimensions, all
+    eight groups of index bits."""
+    rng = np.random.default_rng(5)
+    px, py, idx = (rng.integers(0, m, 512) for m in (2048, 2048, 1024))
+    for k in range(0, 64, 16):  # every draw of a path takes the next dimensions
+        kinds = [1] * k + [3] * (64 - k)
+        ours = device_zsobol(1024, 2048, 2048, px, py, idx, kinds)
+        assert ours.tobytes() == O.zsobol_batch(1024, 2048, 2048, px, py, idx, kinds).tobytes()
