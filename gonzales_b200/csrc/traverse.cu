@@ -1446,24 +1446,26 @@ cudaError_t launch_wide_kernel(TraceKernel k, int stack, bool persistent, bool q
 // lane by lane (k_wide_persistent, k_wide_instanced) instead of through the
 // warp's queue.  Where many rays meet each triangle, neighbouring rays meet it
 // in the same step and the lanes are full as they are: pinhole rays are slower
-// with the queue above about 80 rays a triangle, 400 a node (8.4M rays on 1,280
-// triangles 448 -> 491 us, on 20,480 585 -> 605, on 81,920 681 -> 685; 0.5M on
-// 5,120 83.4 -> 83.9), and faster below (0.5M rays on 20,480 triangles 105.3 ->
-// 101.5, 8.4M on 1,310,720 918 -> 871).  Incoherent rays would be faster with
-// it on small trees too (0.4M on 1,280 triangles 86 -> 77 us), but a launch
-// does not know its rays.
+// with the queue from about 150 rays a node on, by 2 to 3 % at 250 to 500 (4.2M
+// rays on 20,480 triangles 525 -> 547 us, on 81,920 618 -> 625) and by 10 % above
+// 2,000, and faster below (0.5M rays on 81,920 triangles 113 -> 107, 8.4M on
+// 1,310,720 894 -> 876).  Incoherent rays are 5 to 12 % faster with it at every
+// size, but a launch does not know its rays: the line lies where pinhole rays
+// would lose more than 3 %.  A launch that reads its ray count on the device (a
+// renderer's queues) goes by its capacity.
 bool lane_tests(int64_t n, uint32_t nodes) { return n > 400 * (int64_t)nodes; }
 
 template <int RAYFMT, int OUTFMT, bool ANY, int STACK, int LEAF>
 cudaError_t launch_wide_stack(const DevScene &s, const LaunchParams &p, const void *rays, const float *tmax, int64_t n,
                               void *out, cudaStream_t st) {
-        if (p.traversal != GZG_TRAVERSAL_WIDE)
-                return launch_wide_kernel(k_wide<RAYFMT, OUTFMT, ANY, STACK, LEAF>, STACK, false, false, p, s, rays, tmax, n, out, st);
-        // (a tree too deep for 16 entries has too many nodes for the other kernel to matter)
-        if constexpr (STACK <= 16)
-                if (lane_tests(n, s.wide_nodes))
-                        return launch_wide_kernel(k_wide_persistent<RAYFMT, OUTFMT, ANY, STACK, LEAF>, STACK, true, false, p, s,
-                                                  rays, tmax, n, out, st);
+        if constexpr (OUTFMT != kOutShadow)  // (launch_trace takes shadow queues in the persistent kernels only)
+                if (p.traversal != GZG_TRAVERSAL_WIDE)
+                        return launch_wide_kernel(k_wide<RAYFMT, OUTFMT, ANY, STACK, LEAF>, STACK, false, false, p, s, rays, tmax,
+                                                  n, out, st);
+        // (the caller may ask for more entries than the tree needs, so every size has both)
+        if (lane_tests(n, s.wide_nodes))
+                return launch_wide_kernel(k_wide_persistent<RAYFMT, OUTFMT, ANY, STACK, LEAF>, STACK, true, false, p, s, rays,
+                                          tmax, n, out, st);
         return launch_wide_kernel(k_wide_queued<RAYFMT, OUTFMT, ANY, STACK, LEAF>, STACK, true, true, p, s, rays, tmax, n, out, st);
 }
 

@@ -263,3 +263,24 @@ def test_dense_sphere_hits_depend_on_the_ray_alone(leaf):
         torch.cuda.synchronize()
         assert int((got.view(torch.int32) != one.view(torch.int32)).any(1).sum()) == 0
         assert bool((one[:, 3].view(torch.int32) >= 0).any())
+
+
+@pytest.mark.parametrize("depth", [8, 16, 32, 64])
+def test_requested_stack_depth_does_not_choose_the_kernel(depth):
+    """A launch of more than 400 rays a node tests lane by lane whatever stack
+    the caller asks for: node and triangle fetches are those of the kernel that
+    prunes at once (the queue adds some), hits and any hits the same."""
+    import torch
+
+    with GpuAccelerator(_edge_scene("grid", np.random.default_rng(3))) as acc:
+        n = 400 * acc.info()["wide_nodes"] + 777
+        rays = torch.from_numpy(_rays(np.random.default_rng(4), n)).cuda()
+        got = []
+        for o in (dict(traversal=F.TRAVERSAL_WIDE_ONE_RAY_PER_THREAD), dict(stack_depth=depth)):
+            count = torch.zeros(3, dtype=torch.int64, device="cuda")
+            hits = torch.empty((n, 4), device="cuda")
+            acc.trace_closest(rays, hits, options(fetch_counters=count.data_ptr(), **o))
+            torch.cuda.synchronize()
+            got.append((hits.cpu().numpy().tobytes(), count.cpu().tolist()))
+        assert got[0] == got[1]
+        assert acc.error_word() == 0
