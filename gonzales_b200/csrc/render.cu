@@ -476,7 +476,7 @@ struct Wave {
         // second half) or a coated conductor (from its back)
         uint32_t *gen_q;
         uint32_t *counts;      // the bounce's kCountWords counters (the wave's first block outside bounces)
-        int32_t count_blocks;  // blocks of the wave: max_depth + 1
+        int64_t count_blocks;  // blocks of the wave: max_depth + 1
         uint64_t *base;        // first path of the wave
         unsigned long long *stats;  // kStatWords
         // differentiable rendering (single-scene renderers)
@@ -795,7 +795,7 @@ __global__ void k_generate(Wave w) {
         const uint32_t count = wave_count(w);
         const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
         if (blockIdx.x == 0) {
-                for (int k = threadIdx.x; k < w.count_blocks * kCountWords; k += blockDim.x)
+                for (int64_t k = threadIdx.x; k < w.count_blocks * kCountWords; k += blockDim.x)
                         w.counts[k] = k == kCountExt ? count : 0u;
                 if (threadIdx.x == 0) {
                         atomicAdd(w.stats + kStatCamera, (unsigned long long)count);
@@ -1584,7 +1584,7 @@ __global__ void k_probe_resolve(Wave w, DevScene s, int any_only) {
 // Ray statistics of a wave, by one thread after its last bounce.
 __device__ void tally(const Wave &w) {
         unsigned long long ext = 0, shadow = 0, probe = 0;
-        for (int b = 0; b + 1 < w.count_blocks; ++b) {
+        for (int64_t b = 0; b + 1 < w.count_blocks; ++b) {
                 const uint32_t *c = w.counts + b * kCountWords;
                 ext += c[kCountExt];
                 shadow += c[kCountShadow];
@@ -2351,7 +2351,7 @@ gzg_status renderer_create(gzg_scene *const *scenes, const gzg_render_params *pa
         const size_t C = r->max_capacity;
         w.scene_count = (int32_t)n;
         w.count_blocks = 1;
-        for (const gzg_render_params &P : r->params) w.count_blocks = std::max(w.count_blocks, (int32_t)P.max_depth + 1);
+        for (const gzg_render_params &P : r->params) w.count_blocks = std::max(w.count_blocks, (int64_t)P.max_depth + 1);
         const size_t keys = (size_t)std::max<int64_t>(n, r->view.material_count) + 1;
         if (keys > (1u << 20)) return set_error(GZG_ERR_LIMIT, "renderer: more than 2^20 sort keys");
         const SceneConst *scd = nullptr;
