@@ -452,7 +452,7 @@ struct Wave {
         float4 *thr;
         float4 *L;
         uint32_t *pixel;  // batch film pixel
-        uint32_t *scene;
+        uint32_t *scene;  // null with one scene (path_scene)
         float *weight;
         // queues
         float4 *q_ray[2];  // gzg_ray_d, 2 x float4 per entry
@@ -2358,7 +2358,7 @@ gzg_status renderer_create(gzg_scene *const *scenes, const gzg_render_params *pa
         if ((st = r->upload(&scd, r->consts))) return st;
         w.scenes = scd;
         if ((st = r->alloc(&w.zs_morton, C)) || (st = r->alloc(&w.zs_dim, C)) || (st = r->alloc(&w.thr, C)) ||
-            (st = r->alloc(&w.L, C)) || (st = r->alloc(&w.pixel, C)) || (st = r->alloc(&w.scene, C)) ||
+            (st = r->alloc(&w.L, C)) || (st = r->alloc(&w.pixel, C)) || (n > 1 && (st = r->alloc(&w.scene, C))) ||
             (st = r->alloc(&w.weight, C)) || (st = r->alloc(&w.q_ray[0], 2 * C)) || (st = r->alloc(&w.q_ray[1], 2 * C)) ||
             (st = r->alloc(&w.q_id[0], C)) || (st = r->alloc(&w.q_id[1], C)) || (st = r->alloc(&w.hits, C)) ||
             (st = r->alloc(&w.sh_ray, 2 * C)) || (st = r->alloc(&w.sh_id, C)) || (st = r->alloc(&w.sh_contrib, C)) ||

@@ -168,3 +168,21 @@ def test_batch_configuration_subset_matches_oracle():
         helpers.record("batch_subset_vs_oracle.json", record)
         for a in accs:
             a.close()
+
+
+def test_one_scene_keeps_no_scene_index_per_path():
+    """Path state of a renderer: 4 bytes a path more when several scenes share it."""
+    import torch
+
+    accs = [GpuAccelerator(scenes.box_scene().build()) for _ in range(2)]
+    used = []
+    for size, some in ((1024, accs[:1]), (512, accs)):  # 2^22 and 2 x 2^20 paths
+        p = [F.render_params(width=size, height=size, spp=4, max_depth=3) for _ in some]
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        r = BatchRenderer(some, p)
+        used.append((free - torch.cuda.mem_get_info()[0]) / (size * size * 4 * len(some)))
+        r.close()
+    assert used[0] <= used[1] - 3.0
+    for a in accs:
+        a.close()
