@@ -156,51 +156,37 @@ __device__ __noinline__ uint32_t zs_sobol64(const uint32_t *m, uint64_t index) {
         return acc;
 }
 
-// getSampleIndex of N draws of one path at once, in 32-bit arithmetic.  Every
-// base-4 digit of the Morton index is permuted by a hash of the digits above
-// it and the draw's dimension.  mixBits folds its argument to 32 bits by xor,
-// so the argument is (digits above) ^ fold(dim x 0x55555555), and its first
-// step x ^= x >> 16 distributes over that xor: one half is shared by the N
-// draws, the other by the digits.  Only the top byte of the hash is used (its
-// last step leaves that byte alone), and it picks the permutation from the
-// block's table.  About 10 instructions per digit and draw, where hashing each
-// draw on its own with h % 24 and register-selected permutations took 28.  The
-// shade kernels are bound by integer issue, mostly the sampler's: with this, the
-// nibble tables below and no values drawn that nothing reads, the box-scene
-// frame (256 x 256, 16 spp, depth 5) went 1,387 -> 1,108 us, the adjoint step
-// 4.64 -> 3.75 ms, the two-level frame with layered materials 30.9 -> 29.3 ms.
-template <int N>
-__device__ __forceinline__ void zs_index32(const ZSobolConfig &c, uint32_t morton, const ZSlot (&slot)[N],
-                                           uint32_t (&idx)[N]) {
+// getSampleIndex of a draw in 32-bit arithmetic.  Every base-4 digit of the
+// Morton index is permuted by a hash of the digits above it and the draw's
+// dimension.  mixBits folds its argument to 32 bits by xor, so the argument is
+// (digits above) ^ fold(dim x 0x55555555), and its first step x ^= x >> 16
+// distributes over that xor: the dimension's half leaves the loop.  Only the top
+// byte of the hash is used (its last step leaves that byte alone), and it picks
+// the permutation from the block's table.  About 10 instructions per digit, where
+// h % 24 and register-selected permutations took 28.  The shade kernels are bound
+// by integer issue, mostly the sampler's: with this, the nibble tables below and
+// no values drawn that nothing reads, the box-scene frame (256 x 256, 16 spp,
+// depth 5) went 1,387 -> 1,108 us, the adjoint step 4.64 -> 3.75 ms, the two-level
+// frame with layered materials 30.9 -> 29.3 ms.
+__device__ __forceinline__ uint32_t zs_index32(const ZSobolConfig &c, uint32_t morton, int dim) {
         const uint8_t *perm = reinterpret_cast<const uint8_t *>(zs_perm_table());
-        uint32_t fold[N], mixed[N];
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-                const uint64_t dmul = 0x55555555ull * (uint64_t)(int64_t)slot[k].hash;
-                fold[k] = (uint32_t)(dmul & 0xFFFFFFFFull) ^ (uint32_t)(dmul >> 32);
-                mixed[k] = fold[k] ^ (fold[k] >> 16);
-                idx[k] = 0u;
-        }
+        const uint64_t dmul = 0x55555555ull * (uint64_t)(int64_t)dim;
+        const uint32_t fold = (uint32_t)(dmul & 0xFFFFFFFFull) ^ (uint32_t)(dmul >> 32);
+        const uint32_t mixed = fold ^ (fold >> 16);
         const int odd = c.log2spp & 1;
+        uint32_t idx = 0;
 #pragma unroll 1
         for (int shift = 2 * (c.n_base4_digits - 1) - odd; shift >= odd; shift -= 2) {
                 uint32_t above = zs_shr32(morton, shift + 2);
                 above ^= above >> 16;
-                const uint32_t sel = ((morton >> shift) & 3u) * 2u;
-#pragma unroll
-                for (int k = 0; k < N; ++k) {
-                        uint32_t x = (above ^ mixed[k]) * 0x85ebca77u;
-                        x ^= x >> 13;
-                        x *= 0xc2b2ae35u;
-                        const uint32_t e = perm[x >> 24];
-                        idx[k] = idx[k] * 4u + ((e >> sel) & 3u);
-                }
+                uint32_t x = (above ^ mixed) * 0x85ebca77u;
+                x ^= x >> 13;
+                x *= 0xc2b2ae35u;
+                const uint32_t e = perm[x >> 24];
+                idx = idx * 4u + ((e >> (((morton >> shift) & 3u) * 2u)) & 3u);
         }
-        if (odd) {
-#pragma unroll
-                for (int k = 0; k < N; ++k)
-                        idx[k] = idx[k] * 2u + ((morton ^ zs_mix_bits32((morton >> 1) ^ fold[k])) & 1u);
-        }
+        if (odd) idx = idx * 2u + ((morton ^ zs_mix_bits32((morton >> 1) ^ fold)) & 1u);
+        return idx;
 }
 
 // sobolSample's matrix products of `dims` consecutive dimensions from base for
@@ -263,10 +249,7 @@ __device__ __forceinline__ void zs_values(const ZSobolConfig &c, const ZSobol &s
 template <int DIMS>
 __device__ __forceinline__ void zs_draw(const ZSobolConfig &c, const ZSobol &s, const ZSlot &slot, float (&out)[DIMS]) {
         const bool wide = !zs_fits32(c, s);
-        const ZSlot one[1] = {slot};
-        uint32_t idx[1] = {0u};
-        if (!wide) zs_index32<1>(c, (uint32_t)s.morton, one, idx);
-        zs_values<DIMS>(c, s, slot, wide, idx[0], out);
+        zs_values<DIMS>(c, s, slot, wide, wide ? 0u : zs_index32(c, (uint32_t)s.morton, slot.hash), out);
 }
 
 // startPixelSample (ZSobolSampler.swift:130-136).
