@@ -14,10 +14,12 @@ outputs (256 MiB of hits) are larger than the 126 MB L2, so no flush is done.
   e2e       the same through gzg_gpu_traverse_batch (the drop-in call) from
             pinned host Ray_C + tMax to host Intersection_C records
   roofline  algorithmic bytes of the traversal kernel (48 B ray I/O + 80 B per
-            wide node + 48 B per triangle, counts from an instrumented replay)
-            over the average launch time, against the measured HBM copy
-            bandwidth; `coherent` and `incoherent` give the same for each half
-            of the rays launched alone; `io_lower_bound` the ray I/O alone
+            wide node + 48 B per triangle, counts from an instrumented replay
+            of the one-ray-per-thread kernel, which prunes at once) over the
+            average launch time, against the measured HBM copy bandwidth; the
+            timed kernel's own counts stand beside them; `coherent` and
+            `incoherent` give the same for each half of the rays launched alone;
+            `io_lower_bound` the ray I/O alone
             (48 B per ray) and `reference_layout` the bytes the same launch
             time would move in the reference's layout (BVH2 records and
             triangle tests counted by an instrumented replay of the
@@ -651,20 +653,25 @@ def run_ours(args):
     tuned_closest, _ = acc.autotune(rays_d)
     tuned_any, _ = acc.autotune(rays_d, any_hit=True)
 
-    # instrumented replay (untimed): node / triangle fetch counts per launch
+    # instrumented replays (untimed): node / triangle fetches per launch of the
+    # traversal that prunes at once (one ray per thread), which is what the rays
+    # need, and of the timed kernel, whose triangle queue prunes later
     cnt = torch.zeros(3, dtype=torch.int64, device="cuda")
-    acc.trace_closest(rays_d, hits_d, options(fetch_counters=cnt.data_ptr()))
-    torch.cuda.synchronize()
-    nodes_per_launch, tris_per_launch, rays_counted = [int(x) for x in cnt.cpu()]
+
+    def fetches(r, h, **o):
+        cnt.zero_()
+        acc.trace_closest(r, h, options(fetch_counters=cnt.data_ptr(), **o))
+        torch.cuda.synchronize()
+        return [int(x) for x in cnt.cpu()]
+
+    nodes_per_launch, tris_per_launch, rays_counted = fetches(rays_d, hits_d,
+                                                              traversal=F.TRAVERSAL_WIDE_ONE_RAY_PER_THREAD)
     assert rays_counted == n, (rays_counted, n)
+    kernel_nodes, kernel_tris, _ = fetches(rays_d, hits_d)
     # the same rays through the reference's own node order and layout (k_bvh2,
     # untimed): 32-byte BVH2 records fetched (one per iteration, two per
     # interior step) and triangle tests, for the reference-layout bytes
-    from gonzales_b200._ffi import TRAVERSAL_BVH2
-    cnt.zero_()
-    acc.trace_closest(rays_d, hits_d, options(traversal=TRAVERSAL_BVH2, fetch_counters=cnt.data_ptr()))
-    torch.cuda.synchronize()
-    bvh2_records, bvh2_tris, _ = [int(x) for x in cnt.cpu()]
+    bvh2_records, bvh2_tris, _ = fetches(rays_d, hits_d, traversal=F.TRAVERSAL_BVH2)
 
     for _ in range(args.warmup):
         acc.trace_closest(rays_d, hits_d)
@@ -710,10 +717,7 @@ def run_ours(args):
     halves = {}
     for label, sl in (("coherent", slice(0, nc)), ("incoherent", slice(nc, n))):
         rh, hh = rays_d[sl], hits_d[sl]
-        cnt.zero_()
-        acc.trace_closest(rh, hh, options(fetch_counters=cnt.data_ptr()))
-        torch.cuda.synchronize()
-        h_nodes, h_tris, h_rays = [int(x) for x in cnt.cpu()]
+        h_nodes, h_tris, h_rays = fetches(rh, hh, traversal=F.TRAVERSAL_WIDE_ONE_RAY_PER_THREAD)
         for _ in range(args.warmup):
             acc.trace_closest(rh, hh)
         barrier()
@@ -777,9 +781,12 @@ def run_ours(args):
             traffic = json.loads(prof.read_text()).get("dram_bytes_per_full_launch")
         roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                     "frac": achieved / peak, "traffic": traffic, "peak_source": peak_kind,
-                    "kernel": "k_wide_persistent (closest hit)",
+                    # launch_trace's rule: lane by lane above 400 rays per wide node
+                    "kernel": ("k_wide_persistent" if n > 400 * info["wide_nodes"] else "k_wide_queued") + " (closest hit)",
+                    "limited_by": "instruction issue and load latency (profiles/), far below the byte rate",
                     "bytes_per_ray": alg_bytes / n, "nodes_per_ray": nodes_per_launch / n,
-                    "tris_per_ray": tris_per_launch / n}
+                    "tris_per_ray": tris_per_launch / n,
+                    "kernel_nodes_per_ray": kernel_nodes / n, "kernel_tris_per_ray": kernel_tris / n}
         # ray I/O alone (32 B device ray in, 16 B hit out): the lower bound of any layout
         roofline["io_lower_bound"] = {"bytes_per_ray": 48, "achieved": 48.0 * n / avg_launch_s / 1e9,
                                       "frac": 48.0 * n / avg_launch_s / 1e9 / peak}

@@ -7,7 +7,7 @@
 //
 //   generate   Z-Sobol camera sample, Gaussian filter sample, pinhole ray
 //   per bounce b = 0 .. max_depth-1:
-//     extend   closest hit of the extension queue (k_wide_persistent)
+//     extend   closest hit of the extension queue (launch_trace)
 //     [sort]   optional counting sort of the queue by material or scene
 //     shade    emission, light choice + light sample (-> shadow queue),
 //              MIS BSDF sample (-> probe queue, corrected MIS only),
@@ -19,7 +19,7 @@
 //
 // A renderer serves a batch of scenes: each scene has its own camera, film
 // window, sampler, lights and BVH root in a per-scene constant table, every
-// path carries its scene index, and traversal starts at a per-ray root in one
+// path of several scenes carries its scene index, and traversal starts at a per-ray root in one
 // concatenated node array.  A single scene is a batch of one that uses the
 // scene's own device arrays.  Queue lengths live on the device; no stage waits
 // for the host, so a whole wave can be captured as a CUDA graph and replayed.
@@ -1889,8 +1889,8 @@ gzg_status cuda_err(cudaError_t e, const char *what) {
                          std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// Paths per wave unless the caller sets one (about 350 device bytes per path:
-// 5.9 GB at 2^24).  Larger waves keep the later, roulette-thinned bounces
+// Paths per wave unless the caller sets one (about 300 device bytes per path:
+// 5.0 GB at 2^24).  Larger waves keep the later, roulette-thinned bounces
 // wide enough to fill the GPU: the two-level 1920 x 1080 x 64 spp frame takes
 // 1522 / 1316 / 1230 / 1200 ms at 2^21 / 2^22 / 2^23 / 2^24 paths.
 constexpr uint32_t kDefaultWave = 1u << 24;

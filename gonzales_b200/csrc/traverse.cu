@@ -8,11 +8,17 @@
 //   records are fetched as five 128-bit read-only loads; child planes are
 //   8-bit offsets turned into floats with a byte permute.  Leaf triangles are
 //   tested as soon as their node is opened, in leaf order.
+// k_wide_persistent, k_wide_instanced (two levels): the same steps in warps that
+//   stay resident and refill idle lanes.
+// k_wide_queued, k_wide_instanced_queued: those with a warp's triangle tests
+//   gathered in shared memory, one pair of ray and triangle per lane; the default
+//   but for launches of very many rays per node (lane_tests).  All wide kernels
+//   give a ray the same hit.
 // k_bvh2: the host's BVH2 traversed exactly as the reference's
 //   traverse_bvh2_core (kernel.mojo:223-364), one thread per ray, with the
 //   reference's slab arithmetic (kernel.mojo:171-206) in _rn intrinsics.
 //
-// Both kernels are bounded: a step cap equal to the node count (each node is
+// All kernels are bounded: a step cap equal to the node count (each node is
 // visited at most once per ray in a tree) and a stack-depth check set a bit in
 // the scene's error word and end the ray instead of trapping.
 #include "device.cuh"
@@ -330,9 +336,9 @@ __global__ void __launch_bounds__(256) k_wide(DevScene s, const void *__restrict
 // the slowest ray of a fixed 32-ray batch finishes.  Each iteration opens one
 // node and tests its triangles.  A miss reads its tMax again at the end
 // instead of keeping it in a register.
-// Capped at 64 registers (8 blocks of 128 per SM).  With the pull counter the
-// extra warps pay for closest hit's 28 bytes of spills: ray-cast halves
-// against 7 blocks (72 registers, no spills), incoherent 3,170 -> 3,261
+// Capped at 64 registers (8 blocks of 128 per SM; closest hit spills 8 bytes).
+// With the pull counter the extra warps pay (figures of a build that spilled 28):
+// ray-cast halves against 7 blocks (72 registers, no spills), incoherent 3,170 -> 3,261
 // Mrays/s closest and 3,827 -> 4,148 any hit, coherent 8,362 -> 8,456 closest
 // and 9,692 -> 10,197 any hit.  9 blocks (56 registers, 84 bytes of spills)
 // was slower than 7.  On the static schedule 8 blocks was slower than 7.
@@ -577,7 +583,7 @@ __device__ __forceinline__ bool box_before(const DevScene &s, const WideRay &r, 
 
 // Pairs that make a warp test its queue, and rays that only wait for it.  More
 // pairs fill the tests' lanes better but prune later: of 8 to 32 pairs and 2 to
-// 8 rays these were the fastest over camera, incoherent and any-hit rays (8M
+// 8 rays these were the best over camera, incoherent and any-hit rays (8M
 // incoherent rays 1,769 us at 20 pairs and 1,833 at 8 or 32, 8M camera rays 960
 // at 32).
 constexpr int kQueueTests = 12, kQueueWaiting = 3;
@@ -596,10 +602,10 @@ constexpr int kQueueTests = 12, kQueueWaiting = 3;
 // is NaN, or if the watertight test's rounded limit let a t above the limit in.
 // Such a ray starts over with its triangles tested one by one as their node is
 // opened (kAlone), so its hit depends on the ray alone and not on its warp
-// (2 to 3 % of a launch: 8M incoherent rays 1,802 -> 1,841 us, 8M camera rays
-// 869 -> 889).
+// (2 to 3 % of a launch: 8M incoherent rays 1,802 -> 1,849 us, 8M camera rays
+// 870 -> 894).
 // Against k_wide_persistent: 8M incoherent rays on 1,310,720 triangles 2,116 ->
-// 1,841 us, 4M any-hit rays 892 -> 830, 8M camera rays 918 -> 889, 64 x 64 camera
+// 1,849 us, 4M any-hit rays 892 -> 830, 8M camera rays 918 -> 894, 64 x 64 camera
 // rays on 20,480 triangles 41.1 -> 35.9.  launch_trace says where k_wide_persistent stays.
 template <int RAYFMT, int OUTFMT, bool ANY, int STACK, int LEAF>
 __global__ void __launch_bounds__(128, 8) k_wide_queued(DevScene s, const void *__restrict__ rays,

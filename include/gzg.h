@@ -22,6 +22,8 @@
  *   - One scene handle may be used from several host threads at once (the
  *     Gonzales tile renderer calls from cores-1 tasks, TileRenderer.swift:77);
  *     each *_batch call takes its own staging buffers from a locked pool.
+ *     A call on pageable arrays that has the process to itself stages them
+ *     with up to seven helper threads, which end with the call.
  *   - No entry point falls back to a CPU implementation: without a usable
  *     CUDA device they return GZG_ERR_NO_DEVICE.
  */
